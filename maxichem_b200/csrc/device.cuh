@@ -95,6 +95,17 @@ __device__ __forceinline__ Cell cell_arrays(const Net& net, double* smem) {
   return c;
 }
 
+// The thread's index with the CTA's warps rotated by the CTA's place among those of its SM, as CTAs are dealt to the SMs
+// in turn: warp 0 alone runs the triangular solves, and without the rotation every CTA's warp 0 would share one of
+// the SM's four schedulers.
+template <int W>
+__device__ __forceinline__ int spread_tid() {
+  unsigned sms;
+  asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
+  const int turn = (int)(blockIdx.x / sms) * W / 4;
+  return (int)((threadIdx.x + 32 * turn) % (32 * W));
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
@@ -110,6 +121,7 @@ __device__ __forceinline__ double warp_max(double v) {
 // sum of y[0..n) as a warp forms it: lane l adds y[l], y[l + 32], ... then the butterfly (every lane returns it).
 __device__ __forceinline__ double lane_sum(const double* y, int n, int lane) {
   double p = 0.0;
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) p += y[i];
   return warp_sum(p);
 }
@@ -159,9 +171,11 @@ __device__ __forceinline__ void cell_rates(const Net& net, const Cell& c, double
   const double lT = log(Tc), iT = 1.0 / Tc, lKT = log(MX_KB * Tc / MX_P0);
   double* g = c.v;
   const double* cf = net.nasa + (Tc < MX_NASA_SPLIT_T ? 0 : net.ns * 9);
+#pragma unroll 1
   for (int i = tid; i < net.ns; i += nt) g[i] = gibbs_rt(cf + 9 * i, Tc, lT, iT);
   if (tid == 0) g[net.ns] = 0.0;
   __syncthreads();
+#pragma unroll 1
   for (int r = tid; r < net.nr; r += nt) {
     if (r >= net.nrt) {
       c.kf[r] = Jc[r - net.nrt];
@@ -231,6 +245,7 @@ __device__ __forceinline__ double sv_row(const Net& net, const Cell& c, int i) {
 __device__ __forceinline__ double rhs(const Net& net, const Cell& c, const double* Y, bool u0, double nd, int gtid, int gnt, int bar) {
   const int lane = gtid & 31, ns = net.ns;
   const double ntot = lane_sum(Y, ns, lane), xf = nd / ntot, ixf = ntot / nd;
+#pragma unroll 1
   for (int i = gtid; i < ns; i += gnt) c.n[i] = Y[i] * xf;
   if (gtid == 0) {
     c.n[ns] = 1.0;
@@ -238,6 +253,7 @@ __device__ __forceinline__ double rhs(const Net& net, const Cell& c, const doubl
   }
   group_sync(bar, gnt);
   const double* n = c.n;
+#pragma unroll 1
   for (int r = gtid; r < net.nr; r += gnt) {
     const uint64_t w = __ldg(net.rx8 + r);
     const double a = c.kf[r] * n[w & 255] * n[(w >> 8) & 255] * n[(w >> 16) & 255];
@@ -248,6 +264,7 @@ __device__ __forceinline__ double rhs(const Net& net, const Cell& c, const doubl
   sv_pieces_of(net, c, c.v, gtid, gnt);
   group_sync(bar, gnt);
   // each row: its pieces added in order
+#pragma unroll 1
   for (int i = gtid; i < ns; i += gnt) {
     const double r = sv_row(net, c, i);
     c.F[i] = r * ixf;
@@ -265,6 +282,7 @@ __device__ __forceinline__ double rhs(const Net& net, const Cell& c, const doubl
 // A = -Jn (dense, row stride ld), then U = u0 + (-Jn N) / ntot (call.cuh:61-79, jacobian_times_x). Three barriers.
 __device__ __forceinline__ void jacobian_w(const Net& net, const Cell& c, double ntot, int tid, int nt) {
   const int ns = net.ns, ld = net.ld;
+#pragma unroll 1
   for (int i = tid; i < ns * ld; i += nt) c.A[i] = 0.0;
   __syncthreads();
   {  // each thread its entries from its coalesced word stream; the padding words use the zero rate kf[2 nr]
@@ -286,6 +304,7 @@ __device__ __forceinline__ void jacobian_w(const Net& net, const Cell& c, double
     }
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = tid; i < ns; i += nt) {
     const double* a = c.A + i * ld;
     double acc = 0.0;
@@ -295,7 +314,8 @@ __device__ __forceinline__ void jacobian_w(const Net& net, const Cell& c, double
   __syncthreads();
 }
 
-// ---- dense LU without exchanges, blocked (PANEL pivots at a time), with a lookahead of one panel ----
+// ---- dense LU without exchanges, blocked (PANEL pivots at a time), with a lookahead of one panel: the mixed path's
+// FP32 factors (the FP64 ones are lu_mma's) ----
 // Every entry receives its updates A_ij <- fma(-l_ik, A_kj, A_ij) in ascending k, l_ik = A_ik / A_kk taken as
 // A_ik * (1 / A_kk): the order and the operations of the right-looking LU, so the bits of the sparse factorisation
 // on the fill pattern (call.cuh:81-112) for finite data. Per block: the block's pivot rows beyond the panel (one
@@ -363,6 +383,7 @@ __device__ __forceinline__ void panel_warp(T* A, int ld, T* dinv, int kb, int nb
     T piv[PANEL];
 #pragma unroll
     for (int jj = 1; jj < PANEL; jj++) piv[jj] = k + jj < ke ? A[k * ld + k + jj] : T(0);
+#pragma unroll 1
     for (int i = k + 1 + lane; i < ns; i += 32) {
       T* ai = A + i * ld;
       const T l = ai[k] * d;
@@ -407,6 +428,7 @@ __device__ __forceinline__ void lu_factor(const Net& net, T* A, T* dinv, int tid
     __syncthreads();
     const int ken = min(ke + PANEL, ns);
     if (warp == 0) {
+#pragma unroll 1
       for (int i = ke + lane; i < ns; i += 32) {  // panel p + 1's columns, rows ke..
         T* ai = A + i * ld;
         T l[PANEL];
@@ -429,6 +451,175 @@ __device__ __forceinline__ void lu_factor(const Net& net, T* A, T* dinv, int tid
   }
 }
 
+// ---- the FP64 LU on the matrix pipe ----
+// The same factorisation as lu_factor's (the same operations on every entry in ascending pivot order, so the same
+// bits), blocked by 8 with the trailing update as FP64 matrix instructions. mma.m8n8k4 adds its four products to an
+// entry one after the other in ascending k, each a correctly rounded fma: measured equal to the fma chain on 786,432
+// random entries over 24 binary orders of magnitude, at the FP64 pipe's full rate (36.8 TFLOP/s). One instruction does the work of
+// 8 warp-wide fma's, and an 8 x 8 tile needs 8 shared accesses a lane for 512 fma's.
+// Per block: the rows below it (L) on half of the warps and the columns right of it (U) on the other half, one lane
+// each, in registers; then warp 0 updates and factors the next diagonal block while the other warps update the rest.
+// What bounds it now is the chain of the diagonal blocks (69 pivots of a reciprocal, a product, an fma and a shuffle)
+// and shared-memory bandwidth: 69 species, one cell an SM, 25,000 cycles against lu_factor's 60,000, four cells an SM
+// 30,500 against 76,500. The loops are kept rolled where they can be: the whole try is 60 KB of code, and unrolled
+// forms that are faster alone (the diagonal block's pivots, 8-pivot solves) made the call 13 % slower with four cells
+// an SM, by instruction fetch.
+
+// c (8 x 8: lane 4 g + t holds row g, columns 2 t and 2 t + 1) += a (8 x 4: row g, column t) b (4 x 8: row t, column g)
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c0), "+d"(c1) : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ void pair_from(const double* p, double& a, double& b) {
+  a = p[0];
+  b = p[1];
+}
+__device__ __forceinline__ void pair_to(double* p, double a, double b) {
+  p[0] = a;
+  p[1] = b;
+}
+
+// The LU of an 8 x 8 block (its first nb rows and columns) held as mma_f64 holds c, on one warp; 1 / pivot to dinv.
+// The chain from pivot to pivot is a reciprocal, a product and an fma: every lane forms the next pivot alike from
+// values gathered while the reciprocal is under way. An entry that takes no update uses a multiplier or a pivot row's
+// entry of 0, and fma(-0, u, x) = x for finite u.
+__device__ __forceinline__ void lu_diagonal(double& x0, double& x1, double* dinv, int nb, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  double piv = __shfl_sync(FULL, x0, 0);
+  // one pivot k, in column 2 q + S: a the entries of its column's parity, b of the next column's (in lanes t == n)
+  auto pivot = [&](int k, int q, int n, double& a, double& b, bool odd) {
+    const double below = __shfl_sync(FULL, a, 4 * k + 4 + q), right = __shfl_sync(FULL, b, 4 * k + n);
+    const double next = __shfl_sync(FULL, b, 4 * k + 4 + n), col = __shfl_sync(FULL, a, 4 * g + q);
+    const double u0 = __shfl_sync(FULL, x0, 4 * k + t), u1 = __shfl_sync(FULL, x1, 4 * k + t);
+    const double d = rcp_rn(piv);
+    piv = fma(-(below * d), right, next);
+    const double l = col * d, m = g > k ? l : 0.0;
+    x0 = fma(-m, t > q ? u0 : 0.0, x0);
+    x1 = fma(-m, t > q || (t == q && !odd) ? u1 : 0.0, x1);
+    if (t == q && g > k) a = l;
+    if (lane == 0) dinv[k] = d;
+  };
+#pragma unroll 1
+  for (int q = 0; 2 * q < nb; q++) {
+    pivot(2 * q, q, q, x0, x1, false);
+    if (2 * q + 1 < nb) pivot(2 * q + 1, q, q + 1, x1, x0, true);
+  }
+}
+
+// Reads past the matrix's last row or column (a tile's rest) stay inside the cell's shared memory, whose layout keeps
+// (ns + 8) ld + 16 doubles from oA on; such rows and columns of a tile are not written.
+template <int W>
+__device__ __noinline__ void lu_mma(int ns, int ld, int oA, int oD, int tid) {
+  extern __shared__ double smem[];
+  double* A = smem + oA;
+  double* dinv = smem + oD;
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+#pragma unroll 1
+  for (int kb = -8; kb + 8 < ns; kb += 8) {  // the first round only factors the first diagonal block
+    const int ke = kb + 8, m = (ns - ke + 7) >> 3;
+    const double* D = A + kb * ld + kb;
+    if (kb < 0) {
+    } else if (warp < W / 2) {  // L: row i of the block's columns times U^-1
+#pragma unroll 1
+      for (int i = ke + tid; i < ns; i += 16 * W) {
+        double* r = A + i * ld + kb;
+        double x[8];
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) pair_from(r + j, x[j], x[j + 1]);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          x[k] *= dinv[kb + k];
+          double u[8];
+#pragma unroll
+          for (int j = (k + 1) & ~1; j < 8; j += 2) pair_from(D + k * ld + j, u[j], u[j + 1]);
+#pragma unroll
+          for (int j = k + 1; j < 8; j++) x[j] = fma(-x[k], u[j], x[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) pair_to(r + j, x[j], x[j + 1]);
+      }
+    } else {  // U: column j of the block's rows, L^-1 times it
+#pragma unroll 1
+      for (int j = ke + tid - 16 * W; j < ns; j += 16 * W) {
+        double* cj = A + kb * ld + j;
+        double x[8];
+#pragma unroll
+        for (int s = 0; s < 8; s++) x[s] = cj[s * ld];
+#pragma unroll
+        for (int s = 1; s < 8; s++) {
+          double l[8];
+#pragma unroll
+          for (int k = 0; k < s; k += 2) pair_from(D + s * ld + k, l[k], l[k + 1]);
+#pragma unroll
+          for (int k = 0; k < s; k++) x[s] = fma(-l[k], x[k], x[s]);
+          cj[s * ld] = x[s];
+        }
+      }
+    }
+    __syncthreads();
+    // the trailing tiles: warp 0 the first one (the next diagonal block), the other warps the rest by tile rows
+    if (warp == 0) {
+      double* cp = A + (ke + g) * ld + ke + 2 * t;
+      double c0, c1;
+      pair_from(cp, c0, c1);
+      if (kb >= 0) {
+        const double* la = A + (ke + g) * ld + kb + t;
+        const double* ub = A + (kb + t) * ld + ke + g;
+        mma_f64(c0, c1, -la[0], ub[0]);
+        mma_f64(c0, c1, -la[4], ub[4 * ld]);
+      }
+      const int nb = min(8, ns - ke);
+      lu_diagonal(c0, c1, dinv + ke, nb, lane);
+      if (g < nb && 2 * t < nb) cp[0] = c0;
+      if (g < nb && 2 * t + 1 < nb) cp[1] = c1;
+    } else if (kb >= 0) {
+#pragma unroll 1
+      for (int ti = warp - 1; ti < m; ti += W - 1) {
+        const int r0 = ke + 8 * ti + g;
+        const double* la = A + r0 * ld + kb + t;
+        const double a0 = -la[0], a1 = -la[4];
+        const double* ub = A + (kb + t) * ld + ke + g;
+        double* cp = A + r0 * ld + ke + 2 * t;
+        int left = ns - ke - 2 * t;  // columns from the lane's first one on
+        if (r0 >= ns) left = 0;
+        int tj = 0;
+        if (ti == 0) {  // its first tile is warp 0's
+          tj = 1;
+          ub += 8;
+          cp += 8;
+          left -= 8;
+        }
+#pragma unroll 1
+        for (; tj < m; tj += 2) {
+          double c0, c1, e0, e1;
+          pair_from(cp, c0, c1);
+          pair_from(cp + 8, e0, e1);
+          const double b0 = ub[0], f0 = ub[8], b1 = ub[4 * ld], f1 = ub[4 * ld + 8];
+          mma_f64(c0, c1, a0, b0);
+          mma_f64(e0, e1, a0, f0);
+          mma_f64(c0, c1, a1, b1);
+          mma_f64(e0, e1, a1, f1);
+          if (left > 1) pair_to(cp, c0, c1);
+          else if (left > 0) cp[0] = c0;
+          if (left > 9) pair_to(cp + 8, e0, e1);
+          else if (left > 8) cp[8] = e0;
+          ub += 16;
+          cp += 16;
+          left -= 16;
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// the LU of A into A and dinv by the cell's W warps
+template <int W>
+__device__ __forceinline__ void lu(const Net& net, double* A, double* dinv, int tid) {
+  extern __shared__ double smem[];
+  lu_mma<W>(net.ns, net.ld, (int)(A - smem), (int)(dinv - smem), tid);
+}
+
 // value a[p] for p = idx (R known at compile time: no local memory)
 template <int R>
 __device__ __forceinline__ double pick(const double (&a)[R], int idx) {
@@ -439,14 +630,8 @@ __device__ __forceinline__ double pick(const double (&a)[R], int idx) {
   return v;
 }
 
-// y <- M0^-1 y on one warp for NV vectors (1 or 2) with the factors of lu_factor: lane l holds rows l + 32 p.
-// Forward unit L in ascending k, U in descending k with x_k = a_k / U_kk (msolve, common.cuh:504-522). Pivots are
-// taken 32 at a time, so the pivot's value comes from a register chosen at compile time (c) and one shuffle; the next
-// column of L or U is loaded while the current pivot is applied. A lane whose row takes no update from pivot k uses
-// the multiplier 0, and fma(-0, y, a) = a for finite y. Each entry receives the one-pivot sweep's fma's in its order.
-// Not inlined: the call kernel solves at four places, and one copy of the code keeps the instruction cache warm.
 // The forward and backward sweeps of M0^-1 on NV register-held vectors (a: lane l holds rows l + 32 p; d: 1 / U_kk),
-// the body of lu_solve (double) and of the mixed path's solve (float). On return a[v][p] * d[p] is the solution.
+// the body of the mixed path's FP32 solve. On return a[v][p] * d[p] is the solution.
 template <int R, int NV, typename T>
 __device__ __forceinline__ void lu_sweep(const Net& net, const T* A, T (&a)[NV][R], const T (&d)[R], int lane) {
   const int ns = net.ns, ld = net.ld, last = ns - 1;
@@ -502,40 +687,167 @@ __device__ __forceinline__ void lu_sweep(const Net& net, const T* A, T (&a)[NV][
   }
 }
 
-// y <- M0^-1 y on one warp for NV vectors (1 or 2) with the factors of lu_factor: lane l holds rows l + 32 p.
-// Forward unit L in ascending k, U in descending k with x_k = a_k / U_kk (msolve, common.cuh:504-522). Pivots are
-// taken 32 at a time, so the pivot's value comes from a register chosen at compile time (c) and one shuffle; the next
-// column of L or U is loaded while the current pivot is applied. A lane whose row takes no update from pivot k uses
-// the multiplier 0, and fma(-0, y, a) = a for finite y. Each entry receives the one-pivot sweep's fma's in its order.
-// Not inlined: the call kernel solves at four places, and one copy of the code keeps the instruction cache warm.
+// y <- M0^-1 y on one warp for NV vectors (1 or 2) with the factors of the LU: lane l holds rows l + 32 p. Forward unit
+// L in ascending k, U in descending k with x_k = a_k / U_kk (msolve, common.cuh:504-522). Each entry receives the
+// one-pivot sweep's fma's in its order, four pivots at a time: their four values are gathered from their lanes, every
+// lane solves the 4 x 4 block alike (its entries are broadcast reads) and applies the four to its rows, so four
+// pivots cost one shuffle latency instead of four; the matrix's last rows past a multiple of four go one by one. One
+// warp issues it, so its instructions and their latencies are the time: 8,500 cycles at 69 species.
+// Not inlined: the call kernel solves at four places, and one copy of the code keeps the instruction cache warm; the
+// vectors and the matrix are offsets into shared memory, so that its accesses stay shared ones.
+// With oU >= 0 the Sherman-Morrison correction of W = M0 - w 1^T follows on the first vector (sherman's operations).
 template <int R, int NV>
-__device__ __noinline__ void lu_solve(const Net& net, const double* A, const double* dinv, double* y0, double* y1,
-                                         int lane) {
-  const int ns = net.ns;
+__device__ __noinline__ void lu_solve_at(int ns, int ld, int oA, int oD, int o0, int o1, int oU, double c0, int lane) {
+  extern __shared__ double smem[];
+  const double* A = smem + oA;
+  const double* dinv = smem + oD;
+  double* y[2] = {smem + o0, smem + o1};
+  const int last = ns - 1, tail = ns & ~3;  // pivots tail .. last one by one
   double a[NV][R], d[R];
+  const double* row[R];
 #pragma unroll
   for (int p = 0; p < R; p++) {
-    const int i = lane + 32 * p;
-    d[p] = i < ns ? dinv[i] : 0.0;
-    a[0][p] = i < ns ? y0[i] : 0.0;
-    if (NV == 2) a[NV - 1][p] = i < ns ? y1[i] : 0.0;
+    const int i = min(lane + 32 * p, last);
+    row[p] = A + i * ld;
+    d[p] = dinv[i];
+#pragma unroll
+    for (int v = 0; v < NV; v++) a[v][p] = y[v][i];
   }
-  lu_sweep<R, NV, double>(net, A, a, d, lane);
-  __syncwarp();
+  const double* dg = A;  // the block's diagonal
 #pragma unroll
-  for (int p = 0; p < R; p++) {
-    const int i = lane + 32 * p;
-    if (i < ns) {
-      y0[i] = a[0][p] * d[p];
-      if (NV == 2) y1[i] = a[NV - 1][p] * d[p];
+  for (int c = 0; c < R; c++) {  // forward: rows 32 c .. 32 c + 31
+    const int nb = min(32, tail - 32 * c);
+#pragma unroll 1
+    for (int b = 0; b < nb; b += 4) {
+      const int k = 32 * c + b;
+      const double *d1 = dg + ld, *d2 = d1 + ld, *d3 = d2 + ld;
+      const double l10 = d1[0], l20 = d2[0], l21 = d2[1], l30 = d3[0], l31 = d3[1], l32 = d3[2];
+      double l[R][4], g[NV][4];
+#pragma unroll
+      for (int v = 0; v < NV; v++)
+#pragma unroll
+        for (int s = 0; s < 4; s++) g[v][s] = __shfl_sync(FULL, a[v][c], b + s);
+#pragma unroll
+      for (int p = c; p < R; p++)
+#pragma unroll
+        for (int s = 0; s < 4; s++) l[p][s] = row[p][k + s];
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        g[v][1] = fma(-l10, g[v][0], g[v][1]);
+        g[v][2] = fma(-l20, g[v][0], g[v][2]);
+        g[v][3] = fma(-l30, g[v][0], g[v][3]);
+        g[v][2] = fma(-l21, g[v][1], g[v][2]);
+        g[v][3] = fma(-l31, g[v][1], g[v][3]);
+        g[v][3] = fma(-l32, g[v][2], g[v][3]);
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+#pragma unroll
+          for (int p = c; p < R; p++)
+            if (p > c || lane > b + s) a[v][p] = fma(-l[p][s], g[v][s], a[v][p]);
+      }
+      dg = d3 + ld + 4;
+    }
+    if (R <= 4 ? c == R - 1 : c == last >> 5) {
+#pragma unroll 1
+      for (int k = tail; k < last; k++) {
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+          const double yk = __shfl_sync(FULL, a[v][c], k & 31);
+          if (lane > (k & 31)) a[v][c] = fma(-row[c][k], yk, a[v][c]);
+        }
+      }
     }
   }
+#pragma unroll
+  for (int c = R - 1; c >= 0; c--) {  // backward: rows 32 c + 31 .. 32 c
+    if (R <= 4 ? c == R - 1 : c == last >> 5) {
+#pragma unroll 1
+      for (int k = last; k >= tail; k--) {
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+          const double z = __shfl_sync(FULL, a[v][c] * d[c], k & 31);
+#pragma unroll
+          for (int p = 0; p <= c; p++)
+            if (p < c || lane < (k & 31)) a[v][p] = fma(-row[p][k], z, a[v][p]);
+        }
+      }
+    }
+    const int nb = min(32, tail - 32 * c);
+#pragma unroll 1
+    for (int q = 4; q <= nb; q += 4) {
+      const int b = nb - q, k = 32 * c + b;
+      dg -= 4 * ld + 4;
+      const double *e1 = dg + ld, *e2 = e1 + ld;
+      const double u01 = dg[1], u02 = dg[2], u03 = dg[3], u12 = e1[2], u13 = e1[3], u23 = e2[3];
+      const double d0 = dinv[k], d1 = dinv[k + 1], d2 = dinv[k + 2], d3 = dinv[k + 3];
+      double u[R][4], g[NV][4];
+#pragma unroll
+      for (int v = 0; v < NV; v++)
+#pragma unroll
+        for (int s = 0; s < 4; s++) g[v][s] = __shfl_sync(FULL, a[v][c], b + s);
+#pragma unroll
+      for (int p = 0; p <= c; p++)
+#pragma unroll
+        for (int s = 0; s < 4; s++) u[p][s] = row[p][k + s];
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        double z[4];
+        z[3] = g[v][3] * d3;
+        z[2] = fma(-u23, z[3], g[v][2]) * d2;
+        z[1] = fma(-u12, z[2], fma(-u13, z[3], g[v][1])) * d1;
+        z[0] = fma(-u01, z[1], fma(-u02, z[2], fma(-u03, z[3], g[v][0]))) * d0;
+#pragma unroll
+        for (int s = 3; s >= 0; s--)
+#pragma unroll
+          for (int p = 0; p <= c; p++)
+            if (p < c || lane < b + s) a[v][p] = fma(-u[p][s], z[s], a[v][p]);
+      }
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < NV; v++)
+#pragma unroll
+    for (int p = 0; p < R; p++) a[v][p] *= d[p];
+  if (oU >= 0) {
+    const double* u = smem + oU;
+    double s = 0.0;
+#pragma unroll
+    for (int p = 0; p < R; p++)
+      if (lane + 32 * p < ns) s += a[0][p];
+    s = warp_sum(s) * c0;
+#pragma unroll
+    for (int p = 0; p < R; p++) a[0][p] = fma(s, u[min(lane + 32 * p, last)], a[0][p]);
+  }
   __syncwarp();
+#pragma unroll
+  for (int v = 0; v < NV; v++)
+#pragma unroll
+    for (int p = 0; p < R; p++)
+      if (lane + 32 * p < ns) y[v][lane + 32 * p] = a[v][p];
+  __syncwarp();
+}
+
+template <int R, int NV>
+__device__ __forceinline__ void lu_solve(const Net& net, const double* A, const double* dinv, double* y0, double* y1,
+                                         int lane) {
+  extern __shared__ double smem[];
+  const int o0 = (int)(y0 - smem), o1 = NV == 2 ? (int)(y1 - smem) : o0;
+  lu_solve_at<R, NV>(net.ns, net.ld, (int)(A - smem), (int)(dinv - smem), o0, o1, -1, 0.0, lane);
+}
+
+// y <- W^-1 y on one warp: the solve and the Sherman-Morrison correction with u = M0^-1 w and c0 = 1 / (1 - sum u)
+template <int R>
+__device__ __forceinline__ void w_solve(const Net& net, const double* A, const double* dinv, double* y, const double* u,
+                                        double c0, int lane) {
+  extern __shared__ double smem[];
+  const int o = (int)(y - smem);
+  lu_solve_at<R, 1>(net.ns, net.ld, (int)(A - smem), (int)(dinv - smem), o, o, (int)(u - smem), c0, lane);
 }
 
 // y <- y + c0 (sum y) u on one warp (sherman_morrison_update, common.cuh:542-557)
 __device__ __forceinline__ void sherman(const Net& net, double* y, const double* u, double c0, int lane) {
   const double s = lane_sum(y, net.ns, lane) * c0;
+#pragma unroll 1
   for (int i = lane; i < net.ns; i += 32) y[i] = fma(s, u[i], y[i]);
   __syncwarp();
 }
@@ -544,11 +856,13 @@ __device__ __forceinline__ void sherman(const Net& net, double* y, const double*
 
 __device__ __forceinline__ void dense_lu_pivot(const Net& net, double* A, double* dinv, int* pr, int lane) {
   const int ns = net.ns, ld = net.ld;
+#pragma unroll 1
   for (int i = lane; i < ns; i += 32) pr[i] = i;
   __syncwarp();
   for (int k = 0; k < ns; k++) {
     double best = -1.0;
     int bi = ns;
+#pragma unroll 1
     for (int i = k + lane; i < ns; i += 32) {
       const double a = fabs(A[i * ld + k]);
       if (a > best) {
@@ -568,6 +882,7 @@ __device__ __forceinline__ void dense_lu_pivot(const Net& net, double* A, double
     const bool exchange = bi != ns && bi != k && !(fabs(A[k * ld + k]) >= MX_PIVTAU * best);
     __syncwarp();
     if (exchange) {
+#pragma unroll 1
       for (int j = lane; j < ns; j += 32) {
         const double a = A[k * ld + j];
         A[k * ld + j] = A[bi * ld + j];
@@ -582,6 +897,7 @@ __device__ __forceinline__ void dense_lu_pivot(const Net& net, double* A, double
     __syncwarp();
     const double dk = 1.0 / A[k * ld + k];
     if (lane == 0) dinv[k] = dk;
+#pragma unroll 1
     for (int i = k + 1 + lane; i < ns; i += 32) {
       const double l = A[i * ld + k] * dk;
       A[i * ld + k] = l;
@@ -651,6 +967,7 @@ __device__ __forceinline__ double step_factor(double en, bool ok, bool prej, dou
 static __device__ void try_error(const Net& net, const Cell& c, bool first, double rtol, double atol, int lane) {
   double e2 = 0.0, em = 0.0;
   bool nn = true;
+#pragma unroll 1
   for (int i = lane; i < net.ns; i += 32) {
     const double y = c.N[i] + 2.0 * c.K1[i] + c.K3[i] + c.K4[i];
     c.Y[i] = y;
@@ -704,6 +1021,7 @@ static __device__ __noinline__ int check_cell(const Net& net, const double* x0, 
     se[lane < nel ? e : ME + e] = acc;
   }
   bool fin = true;
+#pragma unroll 1
   for (int i = lane; i < ns; i += 32) fin = fin && isfinite(xo[i]);
   const bool xfin = __all_sync(FULL, fin);
   __syncwarp();
@@ -718,6 +1036,7 @@ static __device__ __noinline__ int check_cell(const Net& net, const double* x0, 
   const int c = (xfin ? 0 : GUARD_NONFINITE) | (done ? 0 : GUARD_UNFINISHED) | (drift ? GUARD_DRIFT : 0);
   if (c) return c;
   // (A X A^T)[e][f], f >= e: over species with a_ie and a_if both nonzero (guard.cuh:29-37)
+#pragma unroll 1
   for (int q = lane; q < nel * nel; q += 32) {
     const int e = q / nel, f = q - e * nel;
     if (f >= e) {
@@ -753,6 +1072,7 @@ static __device__ __noinline__ int check_cell(const Net& net, const double* x0, 
     }
   }
   __syncwarp();
+#pragma unroll 1
   for (int i = lane; i < ns; i += 32) {  // g per species (guard.cuh:94-99)
     double gi = 1.0;
     for (int e = 0; e < nel; e++) {
@@ -769,10 +1089,12 @@ static __device__ __noinline__ int check_cell(const Net& net, const double* x0, 
   }
   __syncwarp();
   const double sum = sum_at[0];
+#pragma unroll 1
   for (int i = lane; i < ns; i += 32) xo[i] *= g[i];
   __syncwarp();
   if (!(isfinite(sum) && sum > 0.0)) return GUARD_NONFINITE;
   const double is = 1.0 / sum;
+#pragma unroll 1
   for (int i = lane; i < ns; i += 32) xo[i] *= is;
   __syncwarp();
   return 0;
@@ -784,7 +1106,9 @@ __device__ __forceinline__ void stage_guard_inputs(const Net& net, const Cell& c
                                                    const double** at, const double** xin) {
   const int ns = net.ns, na = ns * net.nel;
   if (na + ns > net.a_doubles) return;
+#pragma unroll 1
   for (int e = tid; e < na; e += nt) c.A[e] = __ldg(net.atoms + e);
+#pragma unroll 1
   for (int i = tid; i < ns; i += nt) c.A[na + i] = x0[i];
   *at = c.A;
   *xin = c.A + na;

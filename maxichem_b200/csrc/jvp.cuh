@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(32 * W, 3) jvp_kernel(const Net net, const Cal
       jacobian_w(net, c, ntot, tid, nt);
       for (int i = tid; i < ns; i += nt) c.A[i * ld + i] += igh;
       __syncthreads();
-      lu_factor<32 * W>(net, c.A, c.dinv, tid);
+      lu<W>(net, c.A, c.dinv, tid);
       if (warp == 0) {
         for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
         __syncwarp();

@@ -30,7 +30,7 @@ template <int W, int R, bool PROF, bool LIST = false>
 __global__ void __launch_bounds__(32 * W, 16 / W) call_kernel(const Net net, const CallArgs a, long long* prof) {
   extern __shared__ double smem[];
   const Cell c = cell_arrays(net, smem);
-  const int tid = (int)threadIdx.x, nt = 32 * W, lane = tid & 31, warp = tid >> 5, ns = net.ns, ld = net.ld;
+  const int tid = spread_tid<W>(), nt = 32 * W, lane = tid & 31, warp = tid >> 5, ns = net.ns, ld = net.ld;
   long long ph[PH_COUNT], t0 = 0;
   if (PROF) {
 #pragma unroll
@@ -90,68 +90,87 @@ __global__ void __launch_bounds__(32 * W, 16 / W) call_kernel(const Net net, con
       const double ha = fmin(s.h, dt - s.t), igh = 1.0 / (GAMMA * ha), ih = 1.0 / ha;
       tries++;
       retries += s.prej ? 1 : 0;
-      // F, u and -Jn at N: a retry after a rejection recomputes those of the rejected try, bit for bit
-      const double ntot = rhs(net, c, c.N, true, nd, tid, nt);
-      jacobian_w(net, c, ntot, tid, nt);
-      for (int i = tid; i < ns; i += nt) c.A[i * ld + i] += igh;  // M0 = I / (gamma h) - Jn
-      __syncthreads();
-      mark(PH_RHS_JAC);
-      lu_factor<32 * W>(net, c.A, c.dinv, tid);
-      mark(PH_LU);
-      if (warp == 0) {  // stage 1: K1 on warp 0 and M0^-1 w on warp 1 (msolve, call.cuh:122-131), then Sherman-Morrison
-        for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
-        __syncwarp();
-        lu_solve<R, 1>(net, c.A, c.dinv, c.K1, nullptr, lane);
-      } else if (warp == 1) {
-        lu_solve<R, 1>(net, c.A, c.dinv, c.U, nullptr, lane);
+      // The three right-hand sides share one copy of their code (the try's code is larger than the instruction caches
+      // close to the schedulers: rolled into one loop, and the small strided loops not unrolled, 166 KB of it became
+      // 60): at N on all warps, at Y3 beside warp 0's stage-2 solve, at Y4 on all warps.
+#pragma unroll 1
+      for (int stage = 0; stage < 3; stage++) {
+        const bool beside = stage == 1;
+        double ntot = 0.0;
+        if (beside && warp == 0)
+          w_solve<R>(net, c.A, c.dinv, c.K2, c.U, c0, lane);
+        else
+          ntot = rhs(net, c, stage == 0 ? c.N : c.Y, stage == 0, nd, beside ? tid - 32 : tid, beside ? nt - 32 : nt,
+                     1);
+        if (stage == 0) {
+          // F, u and -Jn at N: a retry after a rejection recomputes those of the rejected try, bit for bit
+          jacobian_w(net, c, ntot, tid, nt);
+#pragma unroll 1
+          for (int i = tid; i < ns; i += nt) c.A[i * ld + i] += igh;  // M0 = I / (gamma h) - Jn
+          __syncthreads();
+          mark(PH_RHS_JAC);
+          lu<W>(net, c.A, c.dinv, tid);
+          mark(PH_LU);
+          if (warp < 2) {  // stage 1: K1 on warp 0 and M0^-1 w on warp 1 (msolve, call.cuh:122-131)
+            double* y = warp == 0 ? c.K1 : c.U;
+            if (warp == 0) {
+#pragma unroll 1
+              for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
+              __syncwarp();
+            }
+            lu_solve<R, 1>(net, c.A, c.dinv, y, nullptr, lane);
+          }
+          __syncthreads();
+          if (warp == 0) {  // Sherman-Morrison, then stage 2's right side and Y3 = N + 2 K1
+            c0 = 1.0 / (1.0 - lane_sum(c.U, ns, lane));
+            const double sc = lane_sum(c.K1, ns, lane) * c0;
+#pragma unroll 1
+            for (int i = lane; i < ns; i += 32) {
+              const double k1 = fma(sc, c.U[i], c.K1[i]);
+              c.K1[i] = k1;
+              c.K2[i] = fma(RODAS_C21 * ih, k1, c.F[i]);
+              c.Y[i] = c.N[i] + 2.0 * k1;
+            }
+          }
+          __syncthreads();
+          continue;
+        }
+        __syncthreads();
+        if (beside)
+          mark(PH_STAGE12);
+        else
+          mark(PH_STAGE3);
+        if (warp == 0) {  // stage 3 and Y4 = N + 2 K1 + K3, or stage 4, the error and the step's factor
+          double* K = beside ? c.K3 : c.K4;
+#pragma unroll 1
+          for (int i = lane; i < ns; i += 32) {
+            const double k12 = c.K1[i] - c.K2[i];
+            K[i] = fma(ih, beside ? k12 : fma(-RODAS_C43, c.K3[i], k12), c.F[i]);
+          }
+          __syncwarp();
+          w_solve<R>(net, c.A, c.dinv, K, c.U, c0, lane);
+          if (beside) {
+#pragma unroll 1
+            for (int i = lane; i < ns; i += 32) c.Y[i] = c.N[i] + 2.0 * c.K1[i] + c.K3[i];
+          } else {
+            try_error(net, c, s.t == 0.0, a.rtol, a.atol, lane);
+            __syncwarp();
+            const double fac = step_factor(c.red[0], c.red[1] != 0.0, s.prej, s.pen, s.pha, ha);
+            if (lane == 0) c.red[2] = fac;
+          }
+        }
+        __syncthreads();
       }
-      __syncthreads();
-      if (warp == 0) {
-        c0 = 1.0 / (1.0 - lane_sum(c.U, ns, lane));
-        sherman(net, c.K1, c.U, c0, lane);
-      }
-      __syncthreads();
-      for (int i = tid; i < ns; i += nt) {
-        c.K2[i] = fma(RODAS_C21 * ih, c.K1[i], c.F[i]);
-        c.Y[i] = c.N[i] + 2.0 * c.K1[i];
-      }
-      __syncthreads();
-      if (warp == 0) {  // stage 2 on warp 0 while the other warps evaluate F(Y3), Y3 = N + 2 K1
-        lu_solve<R, 1>(net, c.A, c.dinv, c.K2, nullptr, lane);
-        sherman(net, c.K2, c.U, c0, lane);
-      } else {
-        rhs(net, c, c.Y, false, nd, tid - 32, nt - 32, 1);
-      }
-      __syncthreads();
-      mark(PH_STAGE12);
-      if (warp == 0) {  // stage 3
-        for (int i = lane; i < ns; i += 32) c.K3[i] = fma(ih, c.K1[i] - c.K2[i], c.F[i]);
-        __syncwarp();
-        lu_solve<R, 1>(net, c.A, c.dinv, c.K3, nullptr, lane);
-        sherman(net, c.K3, c.U, c0, lane);
-        for (int i = lane; i < ns; i += 32) c.Y[i] = c.N[i] + 2.0 * c.K1[i] + c.K3[i];
-      }
-      __syncthreads();
-      rhs(net, c, c.Y, false, nd, tid, nt);
-      mark(PH_STAGE3);
-      if (warp == 0) {  // stage 4 and the error
-        for (int i = lane; i < ns; i += 32)
-          c.K4[i] = fma(ih, fma(-RODAS_C43, c.K3[i], c.K1[i] - c.K2[i]), c.F[i]);
-        __syncwarp();
-        lu_solve<R, 1>(net, c.A, c.dinv, c.K4, nullptr, lane);
-        sherman(net, c.K4, c.U, c0, lane);
-        try_error(net, c, s.t == 0.0, a.rtol, a.atol, lane);
-      }
-      __syncthreads();
       mark(PH_STAGE4);
       const double en = c.red[0];
       const bool ok = c.red[1] != 0.0;
       if (ok) {
+#pragma unroll 1
         for (int i = tid; i < ns; i += nt) c.N[i] = fmax(c.Y[i], 0.0);
         s.t += ha;
         s.nok += 1.0;
       }
-      const double fac = step_factor(en, ok, s.prej, s.pen, s.pha, ha);
+      const double fac = c.red[2];
       s.h = ha * fac;
       s.prej = !ok;
       s.pen = en;
@@ -370,7 +389,7 @@ __global__ void __launch_bounds__(32 * W) debug_try_kernel(const Net net, const 
   __syncthreads();
   for (int i = tid; i < ns; i += nt) c.A[i * ld + i] += igh;
   __syncthreads();
-  lu_factor<32 * W>(net, c.A, c.dinv, tid);
+  lu<W>(net, c.A, c.dinv, tid);
   for (int e = tid; e < ns * ns; e += nt) o[e] = c.A[(e / ns) * ld + e % ns];
   o += ns * ns;
   for (int i = tid; i < ns; i += nt) o[i] = c.dinv[i];
@@ -448,7 +467,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) time_phases_kernel(const Net n
     __syncthreads();
     u = clock64();
     acc[2] += u - t;
-    lu_factor<32 * W>(net, c.A, c.dinv, tid);
+    lu<W>(net, c.A, c.dinv, tid);
     t = clock64();
     acc[3] += t - u;
     if (warp == 0) {
@@ -583,7 +602,7 @@ void cell_layout(const mx_network* n, Net& net) {
     else
       net.oG = take(guard_scratch(ns));
   }
-  net.doubles = off;
+  net.doubles = std::max(off, net.oA + (ns + 8) * net.ld + 16);  // the LU's tiles read past the matrix's last row
 }
 
 void release(mx_solver* s) {

@@ -173,7 +173,7 @@ __device__ __noinline__ void primal_try(const Net& net, const Cell& c, const Ste
   }
   for (int i = tid; i < ns; i += nt) c.A[i * ld + i] += igh;
   __syncthreads();
-  lu_factor<nt>(net, c.A, c.dinv, tid);
+  lu<W>(net, c.A, c.dinv, tid);
   if (warp == 0) {
     for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
     __syncwarp();
