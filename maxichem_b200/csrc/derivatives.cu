@@ -391,7 +391,8 @@ extern "C" int mx_vjp(mx_solver* s, const double* x, const double* T, const doub
   const int stored = 2 * cap;
   // per CTA: k_bar, c1, c2, the try states, the cell's rate-table cotangents (3 nr)
   const long long slot = ((long long)17 * n0.nr + 2LL * stored * (n0.ns + REC_EXTRA) + 1) & ~1ll;
-  const int nchunks = (int)((std::max<int64_t>(B, 1) + ADJ_CHUNK - 1) / ADJ_CHUNK);
+  const int chunk = adjoint_chunk(B, (int64_t)d->vjp_ctas * s->sms);
+  const int nchunks = (int)((std::max<int64_t>(B, 1) + chunk - 1) / chunk);
   const int grid = (int)std::min<int64_t>(nchunks, (int64_t)d->vjp_ctas * s->sms);
   const int rgrid = (int)std::min<int64_t>(std::max<int64_t>(B, 1), (int64_t)d->vjp_recover_ctas * s->sms);
   rcode = grow_doubles(&d->vjp_scratch, &d->vjp_scratch_doubles, (size_t)std::max(grid, rgrid) * (size_t)slot,
@@ -423,7 +424,7 @@ extern "C" int mx_vjp(mx_solver* s, const double* x, const double* T, const doub
     const CallArgs a{x, T, P, dt, h_in, J, (int)B, rtol, atol, max_steps, x_out, h_out, done, steps, flag, status,
                      count, s->list, nullptr};
     AdjArgs aa{lm, gx, gh, adapt, stored, gx0, gT, gP, gdt, gh0, glm, s->net.nj > 0 ? gJ : nullptr, d->vjp_glc,
-               nchunks, chunk_listed, chunk_queue, nullptr, pos, d->vjp_scratch, slot, d->sp_ptr, d->sp_ent, d->st8};
+               chunk, nchunks, chunk_listed, chunk_queue, nullptr, pos, d->vjp_scratch, slot, d->sp_ptr, d->sp_ent, d->st8};
     d->vjp<<<grid, 32 * WARPS, d->vjp_smem, st>>>(net, a, aa, d->adj_layout);
     // the recovered cells' cotangents get a slot each: size them from the count of listed cells (one small read)
     int listed = 0;
@@ -435,7 +436,7 @@ extern "C" int mx_vjp(mx_solver* s, const double* x, const double* T, const doub
       if (rcode) return rcode;
       aa.gLq = d->vjp_glq;
       d->vjp_recover<<<rgrid, 32 * WARPS, d->vjp_smem, st>>>(net, a, aa, d->adj_layout, MX_REC_STEPS * max_steps);
-      arrh_kernel<<<n0.nr, 32, 0, st>>>(net, a, aa, grc);
+      arrh_kernel<<<n0.nr, ARRH_THREADS, 0, st>>>(net, a, aa, grc);
       e = cudaGetLastError();
     }
   } else if (e == cudaSuccess && grc) {  // an empty batch: the rate table's cotangent is zero (if asked for)

@@ -10,8 +10,8 @@
 // sum_k b_k^T J_N K_k, whose Jacobian part comes reaction by reaction from second products of the concentrations.
 // Species sums gather each species' reaction slots from a table in a fixed order: no atomics enter the arithmetic,
 // so the same inputs give the same bits. The rate cotangents reduce to T, P, the log multipliers and J per cell, and
-// to the rate table's Arrhenius columns: the forward kernel takes cells in fixed chunks of ADJ_CHUNK consecutive
-// cells from its queue and adds each passing cell's contribution to its chunk's partial sum in cell order; a cell the
+// to the rate table's Arrhenius columns: the forward kernel takes cells in chunks of consecutive
+// cells (a number that the batch's size sets, adjoint_chunk) from its queue and adds each passing cell's contribution to its chunk's partial sum in cell order; a cell the
 // recovery redoes leaves its contribution in a slot of its own; a last kernel adds the chunks and those slots in a
 // fixed order.
 #pragma once
@@ -25,7 +25,7 @@ struct AdjArgs {
   int adapt, cap;  // cap: stored try states per cell (2 cap of checkpoints and of segment states)
   double *gx0, *gT, *gP, *gdt, *gh0, *glm, *gJ;
   double* gLc;        // [nr][nchunks][9]: per chunk the rate-table cotangent of its cells that passed the guard
-  int nchunks;
+  int chunk, nchunks;  // cells per chunk (adjoint_chunk), chunks
   int* chunk_listed;  // [nchunks]: 1 when a cell of the chunk went to the recovery
   int* chunk_queue;   // the forward kernel's chunk queue
   double* gLq;        // [listed][nr][3]: a recovered cell's cotangents of ln k0's terms and ln k_inf, by list slot
@@ -67,7 +67,16 @@ __device__ __forceinline__ AdjCell adj_arrays(const AdjLayout& l, double* smem) 
 // per-CTA scratch: k_bar [2 nr], slot contributions c1 [nr][6], c2 [nr][6], try states [2][cap][ns + 8], the cell's
 // cotangents of ln k0's terms and ln k_inf [nr][3]
 constexpr int REC_EXTRA = 8;  // h, t, pen, pha, prej, nok and two spare
-constexpr int ADJ_CHUNK = 64;  // cells per chunk of the rate table's partial sums
+constexpr int ADJ_CHUNK = 64;  // most cells per chunk of the rate table's partial sums
+
+// Cells per chunk for B cells on `slots` resident CTAs: about four chunks a CTA, so that the queue evens out cells of
+// different step counts, and at most ADJ_CHUNK, which bounds the partial sums' memory. 4,096 cells of 69 species: 64
+// cells a chunk filled 64 of the 444 CTAs, 239 ms; 2 a chunk, 51 ms.
+inline int adjoint_chunk(int64_t B, int64_t slots) {
+  const int64_t c = B / (4 * (slots > 0 ? slots : 1));
+  return (int)(c < 1 ? 1 : c > ADJ_CHUNK ? ADJ_CHUNK : c);
+}
+
 __device__ __forceinline__ double* adj_kbar(const Net& net, double* sl) { return sl; }
 __device__ __forceinline__ double* adj_c1(const Net& net, double* sl) { return sl + 2 * net.nr; }
 __device__ __forceinline__ double* adj_c2(const Net& net, double* sl) { return sl + 8 * net.nr; }
@@ -930,7 +939,7 @@ __device__ __forceinline__ void add_to_chunk(const Net& net, const AdjArgs& aa, 
 
 // The adjoint kernel: the call kernel's screening, rates, tries (each try's state stored), output and guard, then,
 // for a cell that passed the guard, the reverse pass and its cotangents. A listed cell is left to the recovery's.
-// Cells come in chunks of ADJ_CHUNK consecutive cells from the queue, each chunk's cells in order, so each chunk's
+// Cells come in chunks of aa.chunk consecutive cells from the queue, each chunk's cells in order, so each chunk's
 // partial sum of the rate table's cotangent is formed by one CTA in a fixed order.
 template <int W, int R>
 __global__ void __launch_bounds__(32 * W, 3) vjp_kernel(const Net net, const CallArgs a, const AdjArgs aa,
@@ -942,7 +951,7 @@ __global__ void __launch_bounds__(32 * W, 3) vjp_kernel(const Net net, const Cal
   double* sl = aa.scratch + (size_t)blockIdx.x * aa.slot;
   int chunk = (int)blockIdx.x;
   while (chunk < aa.nchunks) {
-    const int first_cell = chunk * ADJ_CHUNK, end_cell = min(a.B, first_cell + ADJ_CHUNK);
+    const int first_cell = chunk * aa.chunk, end_cell = min(a.B, first_cell + aa.chunk);
     bool started = false, any_listed = false;
     for (int cell = first_cell; cell < end_cell; cell++) {
       const double Tc = a.T[cell], dt = a.dt[cell], hin = a.h_in[cell], P = a.P[cell];
@@ -1162,28 +1171,41 @@ __global__ void __launch_bounds__(32 * W, 3) vjp_recover_kernel(const Net net, c
   }
 }
 
-// The rate table's cotangent: per reaction (one block of 9 threads, one per column), the chunks' partial sums in
-// chunk order, each chunk followed by its recovered cells in cell order (their list slots' cotangents times 1, ln T,
-// -1 / T); cells that still fail (flag 2) or were refused are left out. Photolysis rows are 0. A fixed order: the
-// same inputs give the same bits, whatever the queues did.
-__global__ void arrh_kernel(const Net net, const CallArgs a, const AdjArgs aa, double* grc) {
+// The rate table's cotangent: per reaction (one block; one thread per column), the chunks' partial sums in chunk order,
+// each chunk followed by its recovered cells in cell order (their list slots' cotangents times 1, ln T, -1 / T); cells
+// that still fail (flag 2) or were refused are left out. Photolysis rows are 0. A fixed order: the same inputs give
+// the same bits, whatever the queues did. The block brings ARRH_TILE chunks at a time into shared memory (their 9
+// doubles are contiguous), so that the sums wait for an add and not for a load per chunk.
+constexpr int ARRH_TILE = 64, ARRH_THREADS = 128;
+__global__ void __launch_bounds__(ARRH_THREADS) arrh_kernel(const Net net, const CallArgs a, const AdjArgs aa, double* grc) {
+  __shared__ double part[9 * ARRH_TILE];
+  __shared__ int listed[ARRH_TILE];
   const int r = (int)blockIdx.x, j = (int)threadIdx.x;
-  if (j >= 9) return;
   double acc = 0.0;
   if (r < net.nrt) {
     const int e = j / 3, kind = j % 3;
-    for (int k = 0; k < aa.nchunks; k++) {
-      acc += aa.gLc[((size_t)r * aa.nchunks + k) * 9 + j];
-      if (!aa.chunk_listed[k]) continue;
-      const int c1 = min(a.B, (k + 1) * ADJ_CHUNK);
-      for (int cell = k * ADJ_CHUNK; cell < c1; cell++) {
-        if (a.flag[cell] != 1) continue;  // passed (in the chunk's sum), still failed or refused
-        const double g = aa.gLq[((size_t)aa.pos[cell] * net.nr + r) * 3 + e], Tc = a.T[cell];
-        acc = kind == 0 ? acc + g : (kind == 1 ? fma(g, log(Tc), acc) : fma(-g, 1.0 / Tc, acc));
+    const double* rows = aa.gLc + (size_t)r * aa.nchunks * 9;
+    for (int k0 = 0; k0 < aa.nchunks; k0 += ARRH_TILE) {
+      const int nk = min(ARRH_TILE, aa.nchunks - k0);
+      for (int q = j; q < 9 * nk; q += ARRH_THREADS) part[q] = rows[(size_t)k0 * 9 + q];
+      for (int q = j; q < nk; q += ARRH_THREADS) listed[q] = aa.chunk_listed[k0 + q];
+      __syncthreads();
+      if (j < 9) {
+        for (int k = 0; k < nk; k++) {
+          acc += part[9 * k + j];
+          if (!listed[k]) continue;
+          const int64_t c0 = (int64_t)(k0 + k) * aa.chunk, c1 = min((int64_t)a.B, c0 + aa.chunk);
+          for (int64_t cell = c0; cell < c1; cell++) {
+            if (a.flag[cell] != 1) continue;  // passed (in the chunk's sum), still failed or refused
+            const double g = aa.gLq[((size_t)aa.pos[cell] * net.nr + r) * 3 + e], Tc = a.T[cell];
+            acc = kind == 0 ? acc + g : (kind == 1 ? fma(g, log(Tc), acc) : fma(-g, 1.0 / Tc, acc));
+          }
+        }
       }
+      __syncthreads();
     }
   }
-  grc[(size_t)r * 9 + j] = acc;
+  if (j < 9) grc[(size_t)r * 9 + j] = acc;
 }
 
 }  // namespace mx
