@@ -506,6 +506,48 @@ __device__ __forceinline__ void lu_diagonal(double& x0, double& x1, double* dinv
   }
 }
 
+// The block kb .. kb + 7 of L and U applied to the trailing tiles of tile rows first, first + step, ... (without_first:
+// all but the first tile of tile row 0) on one warp.
+__device__ __forceinline__ void trailing_tiles(double* A, int ld, int kb, int ns, int first, int step,
+                                               bool without_first, int lane) {
+  const int ke = kb + 8, m = (ns - ke + 7) >> 3, g = lane >> 2, t = lane & 3;
+#pragma unroll 1
+  for (int ti = first; ti < m; ti += step) {
+    const int r0 = ke + 8 * ti + g;
+    const double* la = A + r0 * ld + kb + t;
+    const double a0 = -la[0], a1 = -la[4];
+    const double* ub = A + (kb + t) * ld + ke + g;
+    double* cp = A + r0 * ld + ke + 2 * t;
+    int left = ns - ke - 2 * t;  // columns from the lane's first one on
+    if (r0 >= ns) left = 0;
+    int tj = 0;
+    if (without_first && ti == 0) {
+      tj = 1;
+      ub += 8;
+      cp += 8;
+      left -= 8;
+    }
+#pragma unroll 1
+    for (; tj < m; tj += 2) {
+      double c0, c1, e0, e1;
+      pair_from(cp, c0, c1);
+      pair_from(cp + 8, e0, e1);
+      const double b0 = ub[0], f0 = ub[8], b1 = ub[4 * ld], f1 = ub[4 * ld + 8];
+      mma_f64(c0, c1, a0, b0);
+      mma_f64(e0, e1, a0, f0);
+      mma_f64(c0, c1, a1, b1);
+      mma_f64(e0, e1, a1, f1);
+      if (left > 1) pair_to(cp, c0, c1);
+      else if (left > 0) cp[0] = c0;
+      if (left > 9) pair_to(cp + 8, e0, e1);
+      else if (left > 8) cp[8] = e0;
+      ub += 16;
+      cp += 16;
+      left -= 16;
+    }
+  }
+}
+
 // Reads past the matrix's last row or column (a tile's rest) stay inside the cell's shared memory, whose layout keeps
 // (ns + 8) ld + 16 doubles from oA on; such rows and columns of a tile are not written.
 template <int W>
@@ -573,41 +615,7 @@ __device__ __noinline__ void lu_mma(int ns, int ld, int oA, int oD, int tid) {
       if (g < nb && 2 * t < nb) cp[0] = c0;
       if (g < nb && 2 * t + 1 < nb) cp[1] = c1;
     } else if (kb >= 0) {
-#pragma unroll 1
-      for (int ti = warp - 1; ti < m; ti += W - 1) {
-        const int r0 = ke + 8 * ti + g;
-        const double* la = A + r0 * ld + kb + t;
-        const double a0 = -la[0], a1 = -la[4];
-        const double* ub = A + (kb + t) * ld + ke + g;
-        double* cp = A + r0 * ld + ke + 2 * t;
-        int left = ns - ke - 2 * t;  // columns from the lane's first one on
-        if (r0 >= ns) left = 0;
-        int tj = 0;
-        if (ti == 0) {  // its first tile is warp 0's
-          tj = 1;
-          ub += 8;
-          cp += 8;
-          left -= 8;
-        }
-#pragma unroll 1
-        for (; tj < m; tj += 2) {
-          double c0, c1, e0, e1;
-          pair_from(cp, c0, c1);
-          pair_from(cp + 8, e0, e1);
-          const double b0 = ub[0], f0 = ub[8], b1 = ub[4 * ld], f1 = ub[4 * ld + 8];
-          mma_f64(c0, c1, a0, b0);
-          mma_f64(e0, e1, a0, f0);
-          mma_f64(c0, c1, a1, b1);
-          mma_f64(e0, e1, a1, f1);
-          if (left > 1) pair_to(cp, c0, c1);
-          else if (left > 0) cp[0] = c0;
-          if (left > 9) pair_to(cp + 8, e0, e1);
-          else if (left > 8) cp[8] = e0;
-          ub += 16;
-          cp += 16;
-          left -= 16;
-        }
-      }
+      trailing_tiles(A, ld, kb, ns, warp - 1, W - 1, true, lane);
     }
     __syncthreads();
   }
@@ -852,8 +860,9 @@ __device__ __forceinline__ void sherman(const Net& net, double* y, const double*
   __syncwarp();
 }
 
-// ---- the recovery's dense LU with threshold partial pivoting (recover.cuh:7-82), on one warp ----
+// ---- the recovery's dense LU with threshold partial pivoting (recover.cuh:7-82) ----
 
+// On one warp, for more rows a lane than the blocked form's registers hold.
 __device__ __forceinline__ void dense_lu_pivot(const Net& net, double* A, double* dinv, int* pr, int lane) {
   const int ns = net.ns, ld = net.ld;
 #pragma unroll 1
@@ -907,39 +916,165 @@ __device__ __forceinline__ void dense_lu_pivot(const Net& net, double* A, double
   }
 }
 
+// The same factorisation (its exchanges, its operations in its order, so its bits) by the cell's W warps, 8 columns at a
+// time: warp 0 factors the 8 columns in registers (lane l holds rows l + 32 p, the pivot's column in x[.][0]; they move
+// down by one per pivot), the other columns take its exchanges and their rows of U, one lane each, and the trailing
+// tiles run on the matrix instructions as lu_mma's. A recovery is a chain of thousands of tries of a few cells, so its
+// latency is what the call waits for: 1,000 cells of 41 species over 1e10 s, 19 of them recovered, took 116 ms with one
+// warp eliminating an element at a time, 80 ms so.
+template <int W, int R>
+__device__ __noinline__ void dense_lu_at(int ns, int ld, int oA, int oD, int oP, int oX, int tid) {
+  extern __shared__ double smem[];
+  double* A = smem + oA;
+  double* dinv = smem + oD;
+  int* pr = (int*)smem + oP;
+  int* from = (int*)(smem + oX);  // the row that each pivot of the block came from [8]
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll 1
+  for (int i = tid; i < ns; i += 32 * W) pr[i] = i;
+  __syncthreads();
+#pragma unroll 1
+  for (int kb = 0; kb < ns; kb += 8) {
+    const int nb = min(8, ns - kb), ke = kb + nb;
+    if (warp == 0) {
+      double x[R][8];
+#pragma unroll
+      for (int p = 0; p < R; p++) {
+        const int i = lane + 32 * p;
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[p][j] = i >= kb && i < ns && j < nb ? A[i * ld + kb + j] : 0.0;
+      }
+#pragma unroll 1
+      for (int k = 0; k < nb; k++) {
+        const int row = kb + k;
+        double best = -1.0, own[R], u[8], w[8];
+        int bi = ns;
+#pragma unroll
+        for (int p = 0; p < R; p++) {
+          const int i = lane + 32 * p;
+          const double v = fabs(x[p][0]);
+          if (i >= row && i < ns && v > best) {
+            best = v;
+            bi = i;
+          }
+          own[p] = x[p][0];
+        }
+        {  // the largest magnitude over the warp, ties to the lower row; a NaN is never taken
+          const unsigned long long bits = bi < ns ? __double_as_longlong(best) : 0ull;
+          const unsigned hi = (unsigned)(bits >> 32), lo = (unsigned)bits;
+          const unsigned mh = __reduce_max_sync(FULL, hi);
+          const unsigned ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
+          bi = __reduce_min_sync(FULL, bi < ns && hi == mh && lo == ml ? bi : ns);
+          best = bi < ns ? __longlong_as_double((long long)((unsigned long long)mh << 32 | ml)) : -1.0;
+        }
+        const double akk = __shfl_sync(FULL, pick<R>(own, row >> 5), row & 31);
+        const bool exchange = bi != ns && bi != row && !(fabs(akk) >= MX_PIVTAU * best);
+        const int src = exchange ? bi : row;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          double c[R];
+#pragma unroll
+          for (int p = 0; p < R; p++) c[p] = x[p][j];
+          u[j] = __shfl_sync(FULL, pick<R>(c, src >> 5), src & 31);
+          if (exchange) w[j] = __shfl_sync(FULL, pick<R>(c, row >> 5), row & 31);
+        }
+        if (exchange) {
+#pragma unroll
+          for (int p = 0; p < R; p++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+              if (lane + 32 * p == row) x[p][j] = u[j];
+              if (lane + 32 * p == bi) x[p][j] = w[j];
+            }
+          if (lane < k) {  // the block's finished columns
+            double *a0 = A + row * ld + kb + lane, *a1 = A + bi * ld + kb + lane;
+            const double a = *a0;
+            *a0 = *a1;
+            *a1 = a;
+          }
+          if (lane == 8) {
+            const int q = pr[row];
+            pr[row] = pr[bi];
+            pr[bi] = q;
+          }
+          __syncwarp();
+        }
+        const double d = rcp_rn(u[0]);
+#pragma unroll
+        for (int p = 0; p < R; p++) {
+          const int i = lane + 32 * p;
+          const double l = x[p][0] * d;
+          if (i >= kb && i < ns) A[i * ld + row] = i > row ? l : x[p][0];
+#pragma unroll
+          for (int j = 1; j < 8; j++) x[p][j - 1] = i > row ? fma(-l, u[j], x[p][j]) : x[p][j];
+          x[p][7] = 0.0;
+        }
+        if (lane == 0) {
+          dinv[row] = d;
+          from[k] = src;
+        }
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = tid; q < ns - nb; q += 32 * W) {  // the other columns: the exchanges, and right of the block U's rows
+      const int j = q < kb ? q : q + nb;
+      double* cj = A + j;
+#pragma unroll 1
+      for (int k = 0; k < nb; k++) {
+        const int s = from[k];
+        if (s != kb + k) {
+          const double a = cj[(kb + k) * ld];
+          cj[(kb + k) * ld] = cj[s * ld];
+          cj[s * ld] = a;
+        }
+      }
+      if (j >= ke) {
+        const double* D = A + kb * ld + kb;
+        double x[8];
+#pragma unroll
+        for (int s = 0; s < 8; s++) x[s] = cj[(kb + s) * ld];
+#pragma unroll
+        for (int s = 1; s < 8; s++) {
+#pragma unroll
+          for (int k = 0; k < s; k++) x[s] = fma(-D[s * ld + k], x[k], x[s]);
+          cj[(kb + s) * ld] = x[s];
+        }
+      }
+    }
+    __syncthreads();
+    if (ke < ns) trailing_tiles(A, ld, kb, ns, warp, W, false, lane);
+    __syncthreads();
+  }
+}
+
+// P A = L U of the dense W by the cell's W warps: A, dinv (1 / U_kk) and pr; c.red is scratch
+template <int W, int R>
+__device__ __forceinline__ void dense_lu(const Net& net, const Cell& c, int* pr, int tid) {
+  if constexpr (R <= 4) {
+    extern __shared__ double smem[];
+    dense_lu_at<W, R>(net.ns, net.ld, (int)(c.A - smem), (int)(c.dinv - smem), (int)(pr - (int*)smem),
+                      (int)(c.red - smem), tid);
+  } else {
+    if (tid < 32) dense_lu_pivot(net, c.A, c.dinv, pr, tid);
+    __syncthreads();
+  }
+}
+
+// y <- W^-1 y with the factors of dense_lu on one warp: its rows in the exchanges' order, then lu_solve's sweeps
 template <int R>
-__device__ __forceinline__ void dense_solve(const Net& net, const double* A, const double* dinv, const int* pr, double* y, int lane) {
-  const int ns = net.ns, ld = net.ld;
-  double a[R], d[R];
+__device__ __forceinline__ void dense_solve(const Net& net, const double* A, const double* dinv, const int* pr, double* y,
+                                            int lane) {
+  double a[R];
 #pragma unroll
-  for (int p = 0; p < R; p++) {
-    const int i = lane + 32 * p;
-    a[p] = i < ns ? y[pr[i]] : 0.0;
-    d[p] = i < ns ? dinv[i] : 0.0;
-  }
-  for (int k = 0; k < ns - 1; k++) {
-    const double yk = __shfl_sync(FULL, pick<R>(a, k >> 5), k & 31);
-#pragma unroll
-    for (int p = 0; p < R; p++) {
-      const int i = lane + 32 * p;
-      if (i > k && i < ns) a[p] = fma(-A[i * ld + k], yk, a[p]);
-    }
-  }
-  for (int k = ns - 1; k > 0; k--) {
-    const double z = __shfl_sync(FULL, pick<R>(a, k >> 5) * pick<R>(d, k >> 5), k & 31);
-#pragma unroll
-    for (int p = 0; p < R; p++) {
-      const int i = lane + 32 * p;
-      if (i < k) a[p] = fma(-A[i * ld + k], z, a[p]);
-    }
-  }
+  for (int p = 0; p < R; p++) a[p] = lane + 32 * p < net.ns ? y[pr[lane + 32 * p]] : 0.0;
   __syncwarp();
 #pragma unroll
-  for (int p = 0; p < R; p++) {
-    const int i = lane + 32 * p;
-    if (i < ns) y[i] = a[p] * d[p];
-  }
+  for (int p = 0; p < R; p++)
+    if (lane + 32 * p < net.ns) y[lane + 32 * p] = a[p];
   __syncwarp();
+  lu_solve<R, 1>(net, A, dinv, y, nullptr, lane);
 }
 
 // ---- step control (common.cuh:90-133) ----

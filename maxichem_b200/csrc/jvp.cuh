@@ -842,10 +842,10 @@ __global__ void __launch_bounds__(32 * W, 3) jvp_recover_kernel(const Net net, c
           *p = (i == j ? *p + igh : *p) - c.U[i];
         }
         __syncthreads();
+        dense_lu<W, R>(net, c, pr, tid);
         if (warp == 0) {
           for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
           __syncwarp();
-          dense_lu_pivot(net, c.A, c.dinv, pr, lane);
           dense_solve<R>(net, c.A, c.dinv, pr, c.K1, lane);
           for (int i = lane; i < ns; i += 32) c.K2[i] = fma(RODAS_C21 * ih, c.K1[i], c.F[i]);
           __syncwarp();

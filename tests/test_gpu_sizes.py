@@ -1,0 +1,54 @@
+"""The recovery's blocked factorisation at the sizes where its blocks end, and the adjoint's rate-table sum at the batch
+sizes where its chunks change."""
+
+import numpy as np
+import pytest
+import torch
+
+import invented
+from maxichem_b200.ad import ADSolver
+from maxichem_b200.solver import CudaSolver
+from test_gpu_lu import isomers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("warps", [2, 4])
+@pytest.mark.parametrize("species", [3, 8, 9, 17, 33, 41, 64, 65, 97, 130])
+def test_recovered_cells_match_the_plain_call(gpu, tmp_path, species, warps):
+    net = isomers(tmp_path, species)
+    rng = np.random.default_rng(2)
+    x = rng.uniform(0.1, 1.0, (24, species))
+    t = lambda a: torch.tensor(a, dtype=torch.float64, device=gpu)  # noqa: E731
+    args = [t(x / x.sum(1, keepdims=True)), t(rng.uniform(500.0, 1500.0, 24)), t(np.full(24, 1e4)),
+            t(np.full(24, 1e-3)), t(np.full(24, 1e-7))]  # fmt: skip
+    with CudaSolver(net, gpu, warps=warps) as plain, CudaSolver(net, gpu, warps=warps, drift=0.0) as strict:
+        a = plain.launch(*args)
+        b = strict.launch(*args)  # no drift allowed: rounding alone sends most cells through the recovery
+    assert bool(a.done.all()) and int((b.flag > 0).sum()) > 0
+    again = (b.flag > 0).cpu().numpy()
+    xa, xb = a.x.cpu().numpy()[again], b.x.cpu().numpy()[again]
+    # the same steps with another factorisation of the same matrices: rounding times the stiffness, as between orders
+    # of summation elsewhere (1e-9); the guard's correction of the plain result is of the size of its rounding
+    assert np.abs(xa - xb).max() <= 1e-9 and np.array_equal(a.steps.cpu().numpy()[again], b.steps.cpu().numpy()[again])
+
+
+@pytest.mark.parametrize("cells", [1, 7, 1000, 4001])
+def test_the_rate_tables_cotangent_is_the_sum_over_the_cells(gpu, tmp_path, cells):
+    net, _ = invented.hydrogen(tmp_path)
+    rng = np.random.default_rng(cells)
+    x = rng.uniform(0.1, 1.0, (cells, len(net.species)))
+    t = lambda a: torch.tensor(a, dtype=torch.float64, device=gpu)  # noqa: E731
+    args = [t(x / x.sum(1, keepdims=True)), t(rng.uniform(800.0, 1500.0, cells)), t(np.full(cells, 1e5)),
+            t(np.full(cells, 1e-6)), t(np.full(cells, 1e-9))]  # fmt: skip
+    gx = t(rng.standard_normal(x.shape))
+    with ADSolver(net, gpu) as solver:
+        whole = solver.vjp(*args, gx).cotangents.rc
+        assert bool((solver.flag == 0).all())
+        cuts = [0, cells // 3, cells // 2, cells]
+        parts = [solver.vjp(*(a[i:j].clone() for a in args), gx[i:j].clone()).cotangents.rc
+                 for i, j in zip(cuts, cuts[1:]) if j > i]  # fmt: skip
+    total = torch.stack(parts).sum(0)
+    # another order of the same terms: at most a rounding per cell of the largest partial sum
+    scale = torch.stack(parts).abs().amax(0).clamp_min(1e-300)
+    assert float(((whole - total).abs() / scale).max()) <= cells * 4 * 2.3e-16 * 10
