@@ -37,12 +37,12 @@ struct Net {
   const uint32_t* jac_term;
   double etot, drift;
   // per-thread streams of the S v and Jacobian sums for the CTA (group 0) and its last 96 threads (group 1)
-  int st_threads[2], sv_rounds[2], sv_nrows[2], jac_rounds[2], jac_nents[2], n_pieces;
+  int st_threads[2], sv_rounds[2], jac_rounds, n_pieces;
   const int* sv_row_ptr;
-  const uint16_t* sv[2];
-  const uint16_t* sv_rows[2];
-  const uint32_t* jt[2];
-  const uint16_t* jd[2];
+  // four words of a thread together, group q of thread t at q * threads + t, a spare group at the end
+  const uint4* sv[2];  // S v: reaction | coefficient code << 11 | end of a piece << 13 | the piece << 16
+  const uint4* jt;     // the Jacobian's terms, for the CTA
+  const uint2* jd;     // per term 16 bits: where its entry goes when the term ends it
   // shared-memory layout (offsets in doubles); a_doubles: the matrix region's size in doubles. The mixed-precision
   // layout adds the row scales (oS), the Jacobian's diagonal (oDg), n at the try's state (onN), w (oW), the
   // residual (oR) and a stage's right side (oB); the plain layout leaves them 0.
@@ -118,16 +118,24 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// sum of y[0..n) as a warp forms it: lane l adds y[l], y[l + 32], ... then the butterfly (every lane returns it).
+// sum of y[0..n) as a warp forms it: lane l adds y[l], y[l + 32], ... then the butterfly (every lane returns it). Four
+// loads at a time; past the end it adds 0.
 __device__ __forceinline__ double lane_sum(const double* y, int n, int lane) {
   double p = 0.0;
 #pragma unroll 1
-  for (int i = lane; i < n; i += 32) p += y[i];
+  for (int i = lane; i < n; i += 128) {
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) v[q] = i + 32 * q < n ? y[i + 32 * q] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) p += v[q];
+  }
   return warp_sum(p);
 }
 
+// +1, -1, +2, -2 for the codes 0-3 in c's lowest bits, put together as a double's upper half
 __device__ __forceinline__ double code_coefficient(unsigned c) {
-  return (c & 2u) ? ((c & 1u) ? -2.0 : 2.0) : ((c & 1u) ? -1.0 : 1.0);
+  return __hiloint2double((int)((0x3ff00000u + ((c & 2u) << 19)) | (c << 31)), 0);
 }
 
 // ---- rates (common.cuh:136-242) ----
@@ -211,54 +219,74 @@ __device__ __forceinline__ void cell_rates(const Net& net, const Cell& c, double
 // A barrier over the threads of a group: named barrier id (0 is __syncthreads' own) over n threads.
 __device__ __forceinline__ void group_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
-// S v's pieces into part: each thread of the group its pieces (ascending reactions) from its coalesced word stream;
-// v[nr] = 0 pads. Row i of S v is then part[sv_row_ptr[i]] + ... in order (sv_row of the caller).
+// S v's pieces into part: each thread of the group its pieces (ascending reactions) from its coalesced word stream, four
+// words a load and the next four on their way; v[nr] = 0 pads. The four values are read before the first piece is
+// written, which the compiler could not do by itself (a store between them may alias). Row i of S v is then
+// part[sv_row_ptr[i]] + ... in order. What bounds it is the latency of the chain table word, v, fma, store: 69 species,
+// one cell an SM, a right-hand side took 7,450 cycles and takes 4,430.
 __device__ __forceinline__ void sv_pieces_of(const Net& net, const Cell& c, const double* v, int gtid, int gnt) {
   const int g = gnt == net.st_threads[0] ? 0 : 1;
-  const uint16_t* __restrict__ sw = net.sv[g] + gtid;
-  const uint16_t* __restrict__ sr = net.sv_rows[g] + gtid;
+  const uint4* __restrict__ sw = net.sv[g] + gtid;
   double s = 0.0;
-  int piece = 0;
-  const int rounds = net.sv_rounds[g];
-#pragma unroll 4
-  for (int q = 0; q < rounds; q++) {
-    const unsigned w = __ldg(sw + q * gnt);
-    s = fma(code_coefficient(w >> 11), v[w & 0x7ffu], s);
-    if (w & 0x2000u) {
-      c.part[__ldg(sr + piece * gnt)] = s;
-      s = 0.0;
-      piece++;
+  uint4 next = __ldg(sw);
+#pragma unroll 1
+  for (int q = net.sv_rounds[g]; q > 0; q -= 4) {
+    const unsigned w[4] = {next.x, next.y, next.z, next.w};
+    sw += gnt;
+    next = __ldg(sw);
+    double x[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = v[w[k] & 0x7ffu];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      s = fma(code_coefficient(w[k] >> 11), x[k], s);
+      if (w[k] & 0x2000u) {
+        c.part[w[k] >> 16] = s;
+        s = 0.0;
+      }
     }
   }
 }
 
 // Row i of S v from its pieces, added in order.
-__device__ __forceinline__ double sv_row(const Net& net, const Cell& c, int i) {
-  const int p0 = __ldg(net.sv_row_ptr + i), p1 = __ldg(net.sv_row_ptr + i + 1);
+__device__ __forceinline__ double sv_row(const Cell& c, int p0, int p1) {
   double r = c.part[p0];
+#pragma unroll 1
   for (int p = p0 + 1; p < p1; p++) r += c.part[p];
   return r;
+}
+__device__ __forceinline__ double sv_row(const Net& net, const Cell& c, int i) {
+  return sv_row(c, __ldg(net.sv_row_ptr + i), __ldg(net.sv_row_ptr + i + 1));
 }
 
 // F = (ntot / nd) S v(n) at Y, u0 = S v / nd into U when u0; n = nd Y / ntot. Returns ntot. Run by a group of whole
 // warps (gtid its thread index, gnt its size, synchronised by named barrier bar); three barriers.
 __device__ __forceinline__ double rhs(const Net& net, const Cell& c, const double* Y, bool u0, double nd, int gtid, int gnt, int bar) {
-  const int lane = gtid & 31, ns = net.ns;
+  const int lane = gtid & 31, ns = net.ns, nr = net.nr;
+  // what this thread will read from the tables, on its way while the sum is formed
+  const int p0 = gtid < ns ? __ldg(net.sv_row_ptr + gtid) : 0, p1 = gtid < ns ? __ldg(net.sv_row_ptr + gtid + 1) : 0;
+  uint64_t w0 = gtid < nr ? __ldg(net.rx8 + gtid) : 0, w1 = gtid + gnt < nr ? __ldg(net.rx8 + gtid + gnt) : 0;
   const double ntot = lane_sum(Y, ns, lane), xf = nd / ntot, ixf = ntot / nd;
 #pragma unroll 1
   for (int i = gtid; i < ns; i += gnt) c.n[i] = Y[i] * xf;
   if (gtid == 0) {
     c.n[ns] = 1.0;
-    c.v[net.nr] = 0.0;
+    c.v[nr] = 0.0;
   }
   group_sync(bar, gnt);
   const double* n = c.n;
 #pragma unroll 1
-  for (int r = gtid; r < net.nr; r += gnt) {
-    const uint64_t w = __ldg(net.rx8 + r);
-    const double a = c.kf[r] * n[w & 255] * n[(w >> 8) & 255] * n[(w >> 16) & 255];
-    const double b = c.kr[r] * n[(w >> 24) & 255] * n[(w >> 32) & 255] * n[(w >> 40) & 255];
-    c.v[r] = a - b;
+  for (int r = gtid; r < nr; r += 2 * gnt) {  // two reactions at a time, their values read before either is written
+    const uint64_t u = w0, w = w1;
+    const int r1 = r + gnt < nr ? r + gnt : r, r2 = r + 2 * gnt;
+    if (r2 < nr) w0 = __ldg(net.rx8 + r2);
+    if (r2 + gnt < nr) w1 = __ldg(net.rx8 + r2 + gnt);
+    const double a0 = c.kf[r] * n[u & 255] * n[(u >> 8) & 255] * n[(u >> 16) & 255];
+    const double b0 = c.kr[r] * n[(u >> 24) & 255] * n[(u >> 32) & 255] * n[(u >> 40) & 255];
+    const double a1 = c.kf[r1] * n[w & 255] * n[(w >> 8) & 255] * n[(w >> 16) & 255];
+    const double b1 = c.kr[r1] * n[(w >> 24) & 255] * n[(w >> 32) & 255] * n[(w >> 40) & 255];
+    c.v[r] = a0 - b0;
+    if (r1 > r) c.v[r1] = a1 - b1;
   }
   group_sync(bar, gnt);
   sv_pieces_of(net, c, c.v, gtid, gnt);
@@ -266,7 +294,7 @@ __device__ __forceinline__ double rhs(const Net& net, const Cell& c, const doubl
   // each row: its pieces added in order
 #pragma unroll 1
   for (int i = gtid; i < ns; i += gnt) {
-    const double r = sv_row(net, c, i);
+    const double r = i == gtid ? sv_row(c, p0, p1) : sv_row(net, c, i);
     c.F[i] = r * ixf;
     if (u0) c.U[i] = r / nd;
   }
@@ -282,24 +310,36 @@ __device__ __forceinline__ double rhs(const Net& net, const Cell& c, const doubl
 // A = -Jn (dense, row stride ld), then U = u0 + (-Jn N) / ntot (call.cuh:61-79, jacobian_times_x). Three barriers.
 __device__ __forceinline__ void jacobian_w(const Net& net, const Cell& c, double ntot, int tid, int nt) {
   const int ns = net.ns, ld = net.ld;
-#pragma unroll 1
-  for (int i = tid; i < ns * ld; i += nt) c.A[i] = 0.0;
-  __syncthreads();
-  {  // each thread its entries from its coalesced word stream; the padding words use the zero rate kf[2 nr]
-    const uint32_t* __restrict__ jw = net.jt[0] + tid;
-    const uint16_t* __restrict__ jd = net.jd[0] + tid;
-    const int rounds = net.jac_rounds[0];
-    double acc = 0.0;
-    int e = 0;
+  double2* zero = (double2*)c.A;  // to the even count that the layout rounds the matrix to
 #pragma unroll 4
-    for (int q = 0; q < rounds; q++) {
-      const unsigned w = __ldg(jw + q * nt);
-      const double pr = c.kf[w & 0xfffu] * c.n[(w >> 16) & 255u] * c.n[w >> 24];
-      acc = fma(code_coefficient(w >> 12), pr, acc);
-      if (w & 0x4000u) {
-        c.A[__ldg(jd + e * nt)] = -acc;
-        acc = 0.0;
-        e++;
+  for (int i = tid; i < (ns * ld + 1) / 2; i += nt) zero[i] = make_double2(0.0, 0.0);
+  __syncthreads();
+  {  // each thread its entries from its coalesced word stream, four terms a load (the padding words use the zero rate
+     // kf[2 nr]); the four products are formed before the first entry is written. A term at a time, each waiting for
+     // the store before it, the Jacobian and w of 69 species took 14,800 cycles on one cell an SM; 6,800 so.
+    const uint4* __restrict__ jw = net.jt + tid;
+    const uint2* __restrict__ jd = net.jd + tid;
+    double acc = 0.0;
+    uint4 next = __ldg(jw);
+    uint2 next_to = __ldg(jd);
+#pragma unroll 1
+    for (int q = net.jac_rounds; q > 0; q -= 4) {
+      const unsigned w[4] = {next.x, next.y, next.z, next.w};
+      const unsigned to[4] = {next_to.x & 0xffffu, next_to.x >> 16, next_to.y & 0xffffu, next_to.y >> 16};
+      jw += nt;
+      jd += nt;
+      next = __ldg(jw);
+      next_to = __ldg(jd);
+      double pr[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) pr[k] = c.kf[w[k] & 0xfffu] * c.n[(w[k] >> 16) & 255u] * c.n[w[k] >> 24];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        acc = fma(code_coefficient(w[k] >> 12), pr[k], acc);
+        if (w[k] & 0x4000u) {
+          c.A[to[k]] = -acc;
+          acc = 0.0;
+        }
       }
     }
   }
@@ -308,6 +348,7 @@ __device__ __forceinline__ void jacobian_w(const Net& net, const Cell& c, double
   for (int i = tid; i < ns; i += nt) {
     const double* a = c.A + i * ld;
     double acc = 0.0;
+#pragma unroll 8
     for (int j = 0; j < ns; j++) acc = fma(a[j], c.N[j], acc);
     c.U[i] = c.U[i] + acc / ntot;
   }
@@ -558,7 +599,7 @@ __device__ __noinline__ void lu_mma(int ns, int ld, int oA, int oD, int tid) {
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
 #pragma unroll 1
   for (int kb = -8; kb + 8 < ns; kb += 8) {  // the first round only factors the first diagonal block
-    const int ke = kb + 8, m = (ns - ke + 7) >> 3;
+    const int ke = kb + 8;
     const double* D = A + kb * ld + kb;
     if (kb < 0) {
     } else if (warp < W / 2) {  // L: row i of the block's columns times U^-1
@@ -1099,18 +1140,25 @@ __device__ __forceinline__ double step_factor(double en, bool ok, bool prej, dou
 }
 
 // err of a try on warp 0 (try_error, common.cuh:570-590): Y = N + 2 K1 + K3 + K4; writes en and ok to red[0..1].
-static __device__ void try_error(const Net& net, const Cell& c, bool first, double rtol, double atol, int lane) {
-  double e2 = 0.0, em = 0.0;
+// Lane l takes rows l, l + 32, ..., R of them at most, whose divisions then run side by side.
+template <int R>
+__device__ __forceinline__ void try_error(const Net& net, const Cell& c, bool first, double rtol, double atol, int lane) {
+  double q[R], e2 = 0.0, em = 0.0;
   bool nn = true;
-#pragma unroll 1
-  for (int i = lane; i < net.ns; i += 32) {
+#pragma unroll
+  for (int p = 0; p < R; p++) {
+    const int i = min(lane + 32 * p, net.ns - 1);
+    const bool in = lane + 32 * p < net.ns;
     const double y = c.N[i] + 2.0 * c.K1[i] + c.K3[i] + c.K4[i];
-    c.Y[i] = y;
+    if (in) c.Y[i] = y;
     const double sc = fma(rtol, fmax(fabs(c.N[i]), fabs(y)), atol);
-    const double q = c.K4[i] / sc;
-    e2 = fma(q, q, e2);
-    em = fmax(em, fabs(q));
-    nn = nn && (y >= -atol);
+    q[p] = in ? c.K4[i] / sc : 0.0;
+    nn = nn && (!in || y >= -atol);
+  }
+#pragma unroll
+  for (int p = 0; p < R; p++) {
+    e2 = fma(q[p], q[p], e2);
+    em = fmax(em, fabs(q[p]));
   }
   const double er = sqrt(warp_sum(e2) / net.ns), emx = warp_max(em);
   const double en = (first && isfinite(er)) ? fmax(er, emx) : er;

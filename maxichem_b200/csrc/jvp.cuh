@@ -228,27 +228,10 @@ __device__ __forceinline__ double side2(double a0, double a1, double a2, double 
 
 // y = S z on the CTA (z [nr + 1] with z[nr] = 0), through the call's per-thread S v streams. Two barriers.
 __device__ __forceinline__ void s_apply(const Net& net, const Cell& c, const double* z, double* y, int tid, int nt) {
-  const uint16_t* __restrict__ sw = net.sv[0] + tid;
-  const uint16_t* __restrict__ sr = net.sv_rows[0] + tid;
-  double s = 0.0;
-  int piece = 0;
-  const int rounds = net.sv_rounds[0];
-#pragma unroll 4
-  for (int q = 0; q < rounds; q++) {
-    const unsigned w = __ldg(sw + q * nt);
-    s = fma(code_coefficient(w >> 11), z[w & 0x7ffu], s);
-    if (w & 0x2000u) {
-      c.part[__ldg(sr + piece * nt)] = s;
-      s = 0.0;
-      piece++;
-    }
-  }
+  sv_pieces_of(net, c, z, tid, nt);
   __syncthreads();
   for (int i = tid; i < net.ns; i += nt) {
-    const int p0 = __ldg(net.sv_row_ptr + i), p1 = __ldg(net.sv_row_ptr + i + 1);
-    double r = c.part[p0];
-    for (int p = p0 + 1; p < p1; p++) r += c.part[p];
-    y[i] = r;
+    y[i] = sv_row(net, c, i);
   }
   __syncthreads();
 }
@@ -730,7 +713,7 @@ __global__ void __launch_bounds__(32 * W, 3) jvp_kernel(const Net net, const Cal
         __syncwarp();
         lu_solve<R, 1>(net, c.A, c.dinv, c.K4, nullptr, lane);
         sherman(net, c.K4, c.U, c0, lane);
-        try_error(net, c, s.t == 0.0, a.rtol, a.atol, lane);
+        try_error<R>(net, c, s.t == 0.0, a.rtol, a.atol, lane);
       }
       __syncthreads();
       const double en = c.red[0];
@@ -867,7 +850,7 @@ __global__ void __launch_bounds__(32 * W, 3) jvp_recover_kernel(const Net net, c
             c.K4[i] = fma(ih, fma(-RODAS_C43, c.K3[i], c.K1[i] - c.K2[i]), c.F[i]);
           __syncwarp();
           dense_solve<R>(net, c.A, c.dinv, pr, c.K4, lane);
-          try_error(net, c, s.t == 0.0, a.rtol, a.atol, lane);
+          try_error<R>(net, c, s.t == 0.0, a.rtol, a.atol, lane);
         }
         __syncthreads();
         const double en = c.red[0];

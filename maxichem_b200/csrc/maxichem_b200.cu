@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) call_kernel(const Net net, con
 #pragma unroll 1
             for (int i = lane; i < ns; i += 32) c.Y[i] = c.N[i] + 2.0 * c.K1[i] + c.K3[i];
           } else {
-            try_error(net, c, s.t == 0.0, a.rtol, a.atol, lane);
+            try_error<R>(net, c, s.t == 0.0, a.rtol, a.atol, lane);
             __syncwarp();
             const double fac = step_factor(c.red[0], c.red[1] != 0.0, s.prej, s.pen, s.pha, ha);
             if (lane == 0) c.red[2] = fac;
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) recover_kernel(const Net net, 
             c.K4[i] = fma(ih, fma(-RODAS_C43, c.K3[i], c.K1[i] - c.K2[i]), c.F[i]);
           __syncwarp();
           dense_solve<R>(net, c.A, c.dinv, pr, c.K4, lane);
-          try_error(net, c, s.t == 0.0, a.rtol, a.atol, lane);
+          try_error<R>(net, c, s.t == 0.0, a.rtol, a.atol, lane);
         }
         __syncthreads();
         const double en = c.red[0];
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(32 * W) debug_try_kernel(const Net net, const 
     __syncwarp();
     lu_solve<R, 1>(net, c.A, c.dinv, c.K4, nullptr, lane);
     sherman(net, c.K4, c.U, c0, lane);
-    try_error(net, c, true, rtol, atol, lane);
+    try_error<R>(net, c, true, rtol, atol, lane);
   }
   __syncthreads();
   for (int i = tid; i < ns; i += nt) {
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) time_phases_kernel(const Net n
       sherman(net, c.K2, c.U, 0.5, lane);
       t = clock64();
       acc[6] += t - u;
-      try_error(net, c, true, 1e-3, 1e-25, lane);
+      try_error<R>(net, c, true, 1e-3, 1e-25, lane);
       u = clock64();
       acc[7] += u - t;
     }
@@ -639,6 +639,11 @@ __global__ void add_escalated_kernel(const int* sel_count, long long* escalated)
   if (threadIdx.x == 0) escalated[0] += sel_count[0];
 }
 
+// The place of round q's word of thread t with four consecutive rounds of a thread together, and the words of such a
+// stream: whole groups and a spare one, which a thread's reads ahead may touch.
+inline size_t grouped(int q, int t, int threads) { return ((size_t)(q / 4) * threads + t) * 4 + q % 4; }
+inline size_t grouped_words(int rounds, int threads) { return ((size_t)(rounds + 3) / 4 + 1) * threads * 4; }
+
 }  // namespace
 
 extern "C" int mx_create(const mx_network* n, double drift, int device, mx_solver** out, char* err, size_t errlen) {
@@ -758,13 +763,30 @@ extern "C" int mx_create(const mx_network* n, double drift, int device, mx_solve
     const int t = n->stream_threads[g];
     net.st_threads[g] = t;
     net.sv_rounds[g] = n->sv_rounds[g];
-    net.sv_nrows[g] = n->sv_nrows[g];
-    net.jac_rounds[g] = n->jac_rounds[g];
-    net.jac_nents[g] = n->jac_nents[g];
-    e = upload(s, n->sv_stream[g], (size_t)n->sv_rounds[g] * t, &net.sv[g]);
-    if (e == cudaSuccess) e = upload(s, n->sv_rows[g], (size_t)n->sv_nrows[g] * t, &net.sv_rows[g]);
-    if (e == cudaSuccess) e = upload(s, n->jac_stream[g], (size_t)n->jac_rounds[g] * t, &net.jt[g]);
-    if (e == cudaSuccess) e = upload(s, n->jac_dst[g], (size_t)n->jac_nents[g] * t, &net.jd[g]);
+    // a thread's words with the piece that each one's end writes (sv_rows lists a thread's pieces in turn)
+    std::vector<uint32_t> w(grouped_words(n->sv_rounds[g], t), (uint32_t)nr);
+    for (int i = 0; i < t; i++)
+      for (int q = 0, k = 0; q < n->sv_rounds[g]; q++) {
+        const uint32_t word = n->sv_stream[g][(size_t)q * t + i];
+        const bool end = (word & 0x2000u) != 0 && k < n->sv_nrows[g];
+        w[grouped(q, i, t)] = word | (end ? (uint32_t)n->sv_rows[g][(size_t)k * t + i] << 16 : 0u);
+        k += end ? 1 : 0;
+      }
+    e = upload(s, (const uint4*)w.data(), w.size() / 4, &net.sv[g]);
+  }
+  {
+    const int t = n->stream_threads[0], rounds = n->jac_rounds[0];
+    net.jac_rounds = rounds;
+    std::vector<uint32_t> w(grouped_words(rounds, t), (uint32_t)(2 * nr) | (uint32_t)ns << 16 | (uint32_t)ns << 24);
+    std::vector<uint16_t> to(w.size(), 0);
+    for (int i = 0; i < t; i++)
+      for (int q = 0, k = 0; q < rounds; q++) {
+        const uint32_t word = n->jac_stream[0][(size_t)q * t + i];
+        w[grouped(q, i, t)] = word;
+        if ((word & 0x4000u) && k < n->jac_nents[0]) to[grouped(q, i, t)] = n->jac_dst[0][(size_t)k++ * t + i];
+      }
+    if (e == cudaSuccess) e = upload(s, (const uint4*)w.data(), w.size() / 4, &net.jt);
+    if (e == cudaSuccess) e = upload(s, (const uint2*)to.data(), to.size() / 4, &net.jd);
   }
   if (e != cudaSuccess) {
     set_error(err, errlen, "mx_create: %s", cudaGetErrorString(e));

@@ -79,24 +79,33 @@ __device__ __forceinline__ void jacobian_mixed(const Net& net, const Cell& c, co
   for (int i = tid; i < ns * ld; i += nt) e.A[i] = 0.0f;
   for (int i = tid; i < ns; i += nt) e.Dg[i] = 0.0;
   __syncthreads();
-  const uint32_t* __restrict__ jw = net.jt[0] + tid;
-  const uint16_t* __restrict__ jd = net.jd[0] + tid;
-  const int rounds = net.jac_rounds[0];
+  const uint4* __restrict__ jw = net.jt + tid;
+  const uint2* __restrict__ jd = net.jd + tid;
   double acc = 0.0;
-  int k = 0;
-#pragma unroll 4
-  for (int q = 0; q < rounds; q++) {
-    const unsigned w = __ldg(jw + q * nt);
-    const double pr = c.kf[w & 0xfffu] * c.n[(w >> 16) & 255u] * c.n[w >> 24];
-    acc = fma(code_coefficient(w >> 12), pr, acc);
-    if (w & 0x4000u) {
-      const int dst = __ldg(jd + k * nt);
-      if (dst % (ld + 1) == 0)  // p == q: the diagonal, kept in FP64 until gamma h is added
-        e.Dg[dst / (ld + 1)] = -acc;
-      else
-        e.A[dst] = (float)(-acc);
-      acc = 0.0;
-      k++;
+  uint4 next = __ldg(jw);
+  uint2 next_to = __ldg(jd);
+#pragma unroll 1
+  for (int q = net.jac_rounds; q > 0; q -= 4) {
+    const unsigned w[4] = {next.x, next.y, next.z, next.w};
+    const int to[4] = {(int)(next_to.x & 0xffffu), (int)(next_to.x >> 16), (int)(next_to.y & 0xffffu),
+                       (int)(next_to.y >> 16)};
+    jw += nt;
+    jd += nt;
+    next = __ldg(jw);
+    next_to = __ldg(jd);
+    double pr[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) pr[k] = c.kf[w[k] & 0xfffu] * c.n[(w[k] >> 16) & 255u] * c.n[w[k] >> 24];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      acc = fma(code_coefficient(w[k] >> 12), pr[k], acc);
+      if (w[k] & 0x4000u) {
+        if (to[k] % (ld + 1) == 0)  // p == q: the diagonal, kept in FP64 until gamma h is added
+          e.Dg[to[k] / (ld + 1)] = -acc;
+        else
+          e.A[to[k]] = (float)(-acc);
+        acc = 0.0;
+      }
     }
   }
   __syncthreads();
@@ -364,7 +373,7 @@ __global__ void __launch_bounds__(32 * W, 20 / W)
       __syncthreads();
       worst = fmax(worst, refine<R>(net, c, e, c.K4, e.B, igh, c0, a.rtol, a.atol, sweeps, tid, nt));
       if (warp == 0) {
-        try_error(net, c, s.t == 0.0, a.rtol, a.atol, lane);
+        try_error<R>(net, c, s.t == 0.0, a.rtol, a.atol, lane);
         // an accepted try must be trusted; a rejected one only sets the next try's size
         if (lane == 0) c.red[6] = (sweeps > 0 && c.red[1] != 0.0 && !(worst <= tol)) ? 1.0 : 0.0;
       }
@@ -548,7 +557,7 @@ __global__ void __launch_bounds__(32 * W) mixed_debug_kernel(const Net net, cons
   }
   __syncthreads();
   worst = fmax(worst, refine<R>(net, c, e, c.K4, e.B, igh, c0, rtol, atol, sweeps, tid, nt));
-  if (warp == 0) try_error(net, c, true, rtol, atol, lane);
+  if (warp == 0) try_error<R>(net, c, true, rtol, atol, lane);
   __syncthreads();
   for (int i = tid; i < ns; i += nt) {
     out[i] = c.K1[i];

@@ -175,7 +175,7 @@ __device__ __noinline__ void primal_try(const Net& net, const Cell& c, const Ste
       for (int i = lane; i < ns; i += 32) c.K4[i] = fma(ih, fma(-RODAS_C43, c.K3[i], c.K1[i] - c.K2[i]), c.F[i]);
       __syncwarp();
       dense_solve<R>(net, c.A, c.dinv, pr, c.K4, lane);
-      try_error(net, c, s.t == 0.0, rtol, atol, lane);
+      try_error<R>(net, c, s.t == 0.0, rtol, atol, lane);
     }
     __syncthreads();
     return;
@@ -222,7 +222,7 @@ __device__ __noinline__ void primal_try(const Net& net, const Cell& c, const Ste
     __syncwarp();
     lu_solve<R, 1>(net, c.A, c.dinv, c.K4, nullptr, lane);
     sherman(net, c.K4, c.U, c0, lane);
-    try_error(net, c, s.t == 0.0, rtol, atol, lane);
+    try_error<R>(net, c, s.t == 0.0, rtol, atol, lane);
   }
   __syncthreads();
 }
