@@ -95,14 +95,17 @@ __device__ __forceinline__ Cell cell_arrays(const Net& net, double* smem) {
   return c;
 }
 
-// The thread's index with the CTA's warps rotated by the CTA's place among those of its SM, as CTAs are dealt to the SMs
-// in turn: warp 0 alone runs the triangular solves, and without the rotation every CTA's warp 0 would share one of
-// the SM's four schedulers.
+// The thread's index, with a 2-warp CTA's warps exchanged in every other pair of CTAs of an SM. Warp 0 runs the triangular
+// solves, so the warps 0 of an SM's CTAs should sit on different schedulers. The device gives 4-warp CTAs' warps slots
+// that do (measured: 0 1 2 3, 5 6 7 4, 10 11 8 9, 15 12 13 14; rotating them here put all four on one scheduler, 98
+// against 84 ms for 65,536 cells of 69 species), 2-warp CTAs' ones slots 0 1, 2 3, 4 5, ..., two schedulers of four
+// (39.6 against 38.6 ms for 40,000 cells of 41 species).
 template <int W>
 __device__ __forceinline__ int spread_tid() {
+  if (W != 2) return (int)threadIdx.x;
   unsigned sms;
   asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
-  const int turn = (int)(blockIdx.x / sms) * W / 4;
+  const int turn = (int)(blockIdx.x / sms) / 2;
   return (int)((threadIdx.x + 32 * turn) % (32 * W));
 }
 
