@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import invented
+from maxichem_b200 import coupling
 from maxichem_b200.ad import ADSolver
 from maxichem_b200.solver import CudaSolver
 from test_gpu_lu import isomers
@@ -52,3 +53,21 @@ def test_the_rate_tables_cotangent_is_the_sum_over_the_cells(gpu, tmp_path, cell
     # another order of the same terms: at most a rounding per cell of the largest partial sum
     scale = torch.stack(parts).abs().amax(0).clamp_min(1e-300)
     assert float(((whole - total).abs() / scale).max()) <= cells * 4 * 2.3e-16 * 10
+
+
+@pytest.mark.parametrize("cells", [1, 9, 9473])
+@pytest.mark.parametrize("species", [1, 31, 32, 33, 64, 65, 96, 97, 254])
+def test_conversions_at_the_sizes_where_a_lanes_rows_change(gpu, species, cells):
+    rng = np.random.default_rng(species + cells)
+    q, mw = 10.0 ** rng.uniform(-12.0, 0.0, (cells, species)), rng.uniform(1e-3, 1e-1, species)
+    mass = rng.uniform(0.5, 1.5, cells)
+    t = lambda a: torch.tensor(a, dtype=torch.float64, device=gpu)  # noqa: E731
+    x = coupling.mass_to_mole(t(q), t(mw))
+    back = coupling.mole_to_mass(x, t(mw), t(mass)).cpu().numpy()
+    n = q / mw
+    ref = n / n.sum(1, keepdims=True)
+    xm = ref * mw
+    want = xm * (mass / xm.sum(1))[:, None]
+    # positive sums of at most 254 terms in two orders (254 x 1.1e-16), a few roundings beside
+    for got, exact in ((x.cpu().numpy(), ref), (back, want)):
+        assert np.abs(got - exact).max() <= 6e-14 * exact.max() and (np.abs(got / exact - 1.0) <= 6e-14).all()
