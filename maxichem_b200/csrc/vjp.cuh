@@ -247,10 +247,10 @@ __device__ __forceinline__ void primal_update(const Net& net, const Cell& c, Ste
 
 // ---- transposed solves (one warp) ----
 
-// y <- M0^-T y with the factors of lu_factor (unit L below the diagonal, U on and above it), on one warp: U^T z = y in
+// y <- M0^-T y with the factors of the LU (unit L below the diagonal, U on and above it), on one warp: U^T z = y in
 // ascending pivots (z_k = a_k / U_kk, then a_i -= U_ki z_k for i > k), then L^T x = z in descending pivots
 // (a_i -= L_ki x_k for i < k). Lane l holds rows l + 32 p; row k of the factors is read across the lanes
-// (consecutive addresses). As lu_solve: pivots 32 at a time, the pivot's value from a register chosen at compile
+// (consecutive addresses). As lu_sweep: pivots 32 at a time, the pivot's value from a register chosen at compile
 // time and one shuffle, and the next row loaded while the current pivot is applied; a lane whose row takes no update
 // from pivot k uses the multiplier 0 (fma(-0, z, a) = a for finite z). Each entry takes the one-pivot sweep's fma's in
 // its order.
