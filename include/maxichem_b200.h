@@ -226,10 +226,12 @@ int mx_jvp(mx_solver* s, const double* x, const double* T, const double* P, cons
  * fails (flag 2) has NaN cotangents and is left out of grc, as is a refused cell. Results do not depend on the batch
  * order or on the launch: no atomics enter the arithmetic (grc is summed over fixed chunks of 64 consecutive cells
  * and then over the chunks in order, so it keeps its bits for a given batch). Allocates the adjoint's scratch at the
- * first call and when a call needs more: per CTA 17 nr + 4 cap (ns + 8) doubles, per chunk of 64 cells 9 nr doubles
- * (the chunk's partial sum of the rate table's cotangent: 0.5 GB at 1,048,576 cells of 438 reactions), and 3 nr
- * doubles per cell the recovery redoes; one small host read of the count of those cells (a synchronisation of
- * the stream). Calls run one at a time.
+ * first call and when a call needs more, and keeps it for the solver's life: per CTA 17 nr + 4 cap (ns + 8) doubles, per
+ * chunk of 64 cells 9 nr doubles (the chunk's partial sum of the rate table's cotangent: 0.5 GB at 1,048,576 cells of
+ * 438 reactions), and 3 nr doubles for each cell of a batch of fewer than 256 times the resident CTAs (43 MB at 4,096
+ * cells of 438 reactions, 1.2 GB at most on 444 CTAs; without the room for them the call goes on without them, slower,
+ * with the same bits), of a larger batch for each cell that the recovery redoes, with one small host read of the count
+ * of those cells (a synchronisation of the stream). Calls run one at a time.
  */
 int mx_vjp(mx_solver* s, const double* x, const double* T, const double* P, const double* dt, const double* h_in,
            const double* J, const double* lm, const double* rc, int64_t B, double rtol, double atol, int32_t max_steps,

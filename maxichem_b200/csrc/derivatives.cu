@@ -62,9 +62,9 @@ struct mx_derivatives {
   size_t vjp_scratch_doubles = 0;
   double* vjp_glc = nullptr;  // the rate table's chunk partial sums [nr][chunks][9]
   size_t vjp_glc_doubles = 0;
-  double* vjp_glq = nullptr;  // recovered cells' rate-table cotangents [listed][nr][3]
+  double* vjp_glq = nullptr;  // cells' rate-table cotangents [slots][nr][3]: each cell's, or the recovered cells'
   size_t vjp_glq_doubles = 0;
-  int* vjp_ints = nullptr;    // chunk flags [chunks], the chunk queue [1], list slots [B]
+  int* vjp_ints = nullptr;    // chunk flags [chunks], the queue [1], listed cells' slots [B]
   size_t vjp_ints_count = 0;
 };
 
@@ -391,9 +391,16 @@ extern "C" int mx_vjp(mx_solver* s, const double* x, const double* T, const doub
   const int stored = 2 * cap;
   // per CTA: k_bar, c1, c2, the try states, the cell's rate-table cotangents (3 nr)
   const long long slot = ((long long)17 * n0.nr + 2LL * stored * (n0.ns + REC_EXTRA) + 1) & ~1ll;
-  const int chunk = adjoint_chunk(B, (int64_t)d->vjp_ctas * s->sms);
-  const int nchunks = (int)((std::max<int64_t>(B, 1) + chunk - 1) / chunk);
-  const int grid = (int)std::min<int64_t>(nchunks, (int64_t)d->vjp_ctas * s->sms);
+  const int64_t slots = (int64_t)d->vjp_ctas * s->sms, cells = std::max<int64_t>(B, 1);
+  const int nchunks = (int)((cells + ADJ_CHUNK - 1) / ADJ_CHUNK);
+  int run = adjoint_run(nchunks, slots);
+  if (run == 1 && grow_doubles(&d->vjp_glq, &d->vjp_glq_doubles, (size_t)cells * n0.nr * 3,
+                               "cells' rate-table cotangents", err, errlen) != MX_OK) {
+    cudaGetLastError();  // no room for a slot a cell: runs of a chunk give the same sums without them
+    run = ADJ_CHUNK;
+  }
+  const int nruns = run == 1 ? (int)cells : nchunks;
+  const int grid = (int)std::min<int64_t>(nruns, slots);
   const int rgrid = (int)std::min<int64_t>(std::max<int64_t>(B, 1), (int64_t)d->vjp_recover_ctas * s->sms);
   rcode = grow_doubles(&d->vjp_scratch, &d->vjp_scratch_doubles, (size_t)std::max(grid, rgrid) * (size_t)slot,
                        "adjoint scratch", err, errlen);
@@ -413,29 +420,37 @@ extern "C" int mx_vjp(mx_solver* s, const double* x, const double* T, const doub
     d->vjp_ints_count = ints;
   }
   int* chunk_listed = d->vjp_ints;
-  int* chunk_queue = d->vjp_ints + nchunks;
-  int* pos = chunk_queue + 1;
+  int* run_queue = d->vjp_ints + nchunks;
+  int* pos = run_queue + 1;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(count, 0, MX_COUNT_SLOTS * sizeof(int32_t), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(chunk_queue, 0, sizeof(int), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(run_queue, 0, sizeof(int), st);
   if (e == cudaSuccess && B > 0) {
     Net net = s->net;
     if (rc) net.rc = rc;  // the caller's rate table
     const CallArgs a{x, T, P, dt, h_in, J, (int)B, rtol, atol, max_steps, x_out, h_out, done, steps, flag, status,
                      count, s->list, nullptr};
     AdjArgs aa{lm, gx, gh, adapt, stored, gx0, gT, gP, gdt, gh0, glm, s->net.nj > 0 ? gJ : nullptr, d->vjp_glc,
-               chunk, nchunks, chunk_listed, chunk_queue, nullptr, pos, d->vjp_scratch, slot, d->sp_ptr, d->sp_ent, d->st8};
+               run, nruns, nchunks, chunk_listed, run_queue, d->vjp_glq, pos, d->vjp_scratch, slot, d->sp_ptr,
+               d->sp_ent, d->st8};
     d->vjp<<<grid, 32 * WARPS, d->vjp_smem, st>>>(net, a, aa, d->adj_layout);
-    // the recovered cells' cotangents get a slot each: size them from the count of listed cells (one small read)
-    int listed = 0;
-    e = cudaMemcpyAsync(&listed, count + MX_COUNT_RECOMPUTED, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (run != 1) {
+      // the recovered cells' cotangents get a slot each: size them from the count of listed cells (one small read)
+      int listed = 0;
+      e = cudaMemcpyAsync(&listed, count + MX_COUNT_RECOMPUTED, sizeof(int), cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+      if (e == cudaSuccess) {
+        rcode = grow_doubles(&d->vjp_glq, &d->vjp_glq_doubles, (size_t)std::max(listed, 1) * n0.nr * 3,
+                             "recovered cells' rate-table cotangents", err, errlen);
+        if (rcode) return rcode;
+        aa.gLq = d->vjp_glq;
+      }
+    }
     if (e == cudaSuccess) {
-      rcode = grow_doubles(&d->vjp_glq, &d->vjp_glq_doubles, (size_t)std::max(listed, 1) * n0.nr * 3,
-                           "the recovered cells' rate-table cotangents", err, errlen);
-      if (rcode) return rcode;
-      aa.gLq = d->vjp_glq;
       d->vjp_recover<<<rgrid, 32 * WARPS, d->vjp_smem, st>>>(net, a, aa, d->adj_layout, MX_REC_STEPS * max_steps);
+      if (run == 1)
+        chunk_sums_kernel<<<dim3((unsigned)nchunks, (unsigned)((n0.nr + SUMS_THREADS - 1) / SUMS_THREADS)),
+                            SUMS_THREADS, 0, st>>>(net, a, aa);
       arrh_kernel<<<n0.nr, ARRH_THREADS, 0, st>>>(net, a, aa, grc);
       e = cudaGetLastError();
     }

@@ -10,10 +10,10 @@
 // sum_k b_k^T J_N K_k, whose Jacobian part comes reaction by reaction from second products of the concentrations.
 // Species sums gather each species' reaction slots from a table in a fixed order: no atomics enter the arithmetic,
 // so the same inputs give the same bits. The rate cotangents reduce to T, P, the log multipliers and J per cell, and
-// to the rate table's Arrhenius columns: the forward kernel takes cells in chunks of consecutive
-// cells (a number that the batch's size sets, adjoint_chunk) from its queue and adds each passing cell's contribution to its chunk's partial sum in cell order; a cell the
-// recovery redoes leaves its contribution in a slot of its own; a last kernel adds the chunks and those slots in a
-// fixed order.
+// to the rate table's Arrhenius columns: a partial sum per fixed chunk of ADJ_CHUNK consecutive cells, of its passing
+// cells in cell order; a last kernel adds the chunks in order, each followed by its recovered cells. Where a batch has
+// enough chunks for the device, a CTA takes a chunk from the queue and keeps its sum; below that it takes one cell,
+// leaves the cell's contribution in a slot of its own, and chunk_sums_kernel forms the same sums (adjoint_run).
 #pragma once
 #include "jvp.cuh"
 
@@ -25,11 +25,12 @@ struct AdjArgs {
   int adapt, cap;  // cap: stored try states per cell (2 cap of checkpoints and of segment states)
   double *gx0, *gT, *gP, *gdt, *gh0, *glm, *gJ;
   double* gLc;        // [nr][nchunks][9]: per chunk the rate-table cotangent of its cells that passed the guard
-  int chunk, nchunks;  // cells per chunk (adjoint_chunk), chunks
+  int run, nruns, nchunks;  // cells of a queue item (adjoint_run: 1 or ADJ_CHUNK), items, chunks of ADJ_CHUNK cells
   int* chunk_listed;  // [nchunks]: 1 when a cell of the chunk went to the recovery
-  int* chunk_queue;   // the forward kernel's chunk queue
-  double* gLq;        // [listed][nr][3]: a recovered cell's cotangents of ln k0's terms and ln k_inf, by list slot
-  int* pos;           // [B]: a listed cell's slot in the recovery's list
+  int* run_queue;     // the forward kernel's queue
+  double* gLq;        // [slots][nr][3]: a cell's cotangents of ln k0's terms and ln k_inf. run 1: each cell's, by cell;
+                      // else a recovered cell's, by list slot
+  int* pos;           // [B]: a listed cell's slot in gLq
   double* scratch;
   long long slot;
   const int *sp_ptr, *sp_ent;  // species gather: species j's reaction slots sp_ent[sp_ptr[j] .. sp_ptr[j + 1]) = r*8 + m
@@ -67,15 +68,12 @@ __device__ __forceinline__ AdjCell adj_arrays(const AdjLayout& l, double* smem) 
 // per-CTA scratch: k_bar [2 nr], slot contributions c1 [nr][6], c2 [nr][6], try states [2][cap][ns + 8], the cell's
 // cotangents of ln k0's terms and ln k_inf [nr][3]
 constexpr int REC_EXTRA = 8;  // h, t, pen, pha, prej, nok and two spare
-constexpr int ADJ_CHUNK = 64;  // most cells per chunk of the rate table's partial sums
+constexpr int ADJ_CHUNK = 64;  // cells per chunk of the rate table's partial sums: part of the result's definition
 
-// Cells per chunk for B cells on `slots` resident CTAs: about four chunks a CTA, so that the queue evens out cells of
-// different step counts, and at most ADJ_CHUNK, which bounds the partial sums' memory. 4,096 cells of 69 species: 64
-// cells a chunk filled 64 of the 444 CTAs, 239 ms; 2 a chunk, 51 ms.
-inline int adjoint_chunk(int64_t B, int64_t slots) {
-  const int64_t c = B / (4 * (slots > 0 ? slots : 1));
-  return (int)(c < 1 ? 1 : c > ADJ_CHUNK ? ADJ_CHUNK : c);
-}
+// Cells of a queue item for a batch of so many chunks on `slots` resident CTAs: a chunk where each CTA gets at least
+// four, so that the queue evens out cells of different step counts, else one cell, whose contribution waits in
+// 3 nr doubles of its own. 4,096 cells of 69 species: 64 cells an item keep 64 of the 444 CTAs busy, 239 ms; one, 48 ms.
+inline int adjoint_run(int64_t nchunks, int64_t slots) { return nchunks < 4 * slots ? 1 : ADJ_CHUNK; }
 
 __device__ __forceinline__ double* adj_kbar(const Net& net, double* sl) { return sl; }
 __device__ __forceinline__ double* adj_c1(const Net& net, double* sl) { return sl + 2 * net.nr; }
@@ -939,8 +937,8 @@ __device__ __forceinline__ void add_to_chunk(const Net& net, const AdjArgs& aa, 
 
 // The adjoint kernel: the call kernel's screening, rates, tries (each try's state stored), output and guard, then,
 // for a cell that passed the guard, the reverse pass and its cotangents. A listed cell is left to the recovery's.
-// Cells come in chunks of aa.chunk consecutive cells from the queue, each chunk's cells in order, so each chunk's
-// partial sum of the rate table's cotangent is formed by one CTA in a fixed order.
+// Cells come in runs of aa.run consecutive cells from the queue, each run's cells in order: a chunk's partial sum of
+// the rate table's cotangent is formed by the CTA that has the chunk, or from its cells' slots by chunk_sums_kernel.
 template <int W, int R>
 __global__ void __launch_bounds__(32 * W, 3) vjp_kernel(const Net net, const CallArgs a, const AdjArgs aa,
                                                         const AdjLayout al) {
@@ -949,9 +947,9 @@ __global__ void __launch_bounds__(32 * W, 3) vjp_kernel(const Net net, const Cal
   const AdjCell b = adj_arrays(al, smem);
   const int tid = (int)threadIdx.x, nt = 32 * W, lane = tid & 31, warp = tid >> 5, ns = net.ns;
   double* sl = aa.scratch + (size_t)blockIdx.x * aa.slot;
-  int chunk = (int)blockIdx.x;
-  while (chunk < aa.nchunks) {
-    const int first_cell = chunk * aa.chunk, end_cell = min(a.B, first_cell + aa.chunk);
+  int item = (int)blockIdx.x;
+  while (item < aa.nruns) {
+    const int first_cell = item * aa.run, end_cell = (int)min((int64_t)a.B, (int64_t)first_cell + aa.run);
     bool started = false, any_listed = false;
     for (int cell = first_cell; cell < end_cell; cell++) {
       const double Tc = a.T[cell], dt = a.dt[cell], hin = a.h_in[cell], P = a.P[cell];
@@ -1055,7 +1053,12 @@ __global__ void __launch_bounds__(32 * W, 3) vjp_kernel(const Net net, const Cal
         }
         finish_cell(net, c, b, aa, sl, cell, Tc, P, nd, hin, dt, 0, sb, st != 0, c.v, b.Nn, tid, nt);
         if (st == 0) {  // a refused cell stays out of the rate table's sum
-          add_to_chunk(net, aa, sl, chunk, Tc, !started, tid, nt);
+          if (aa.run == 1) {
+            const double* gl = adj_gl(net, aa, sl);
+            for (int e = tid; e < 3 * net.nr; e += nt) aa.gLq[(size_t)cell * 3 * net.nr + e] = gl[e];
+          } else {
+            add_to_chunk(net, aa, sl, item, Tc, !started, tid, nt);
+          }
           started = true;
         }
       } else {
@@ -1063,16 +1066,16 @@ __global__ void __launch_bounds__(32 * W, 3) vjp_kernel(const Net net, const Cal
       }
       __syncthreads();
     }
-    if (!started)  // no passing cell: the chunk's partial sum is zero
+    if (aa.run != 1 && !started)  // no passing cell: the chunk's partial sum is zero
       for (int r = tid; r < net.nr; r += nt)
-        for (int k = 0; k < 9; k++) aa.gLc[((size_t)r * aa.nchunks + chunk) * 9 + k] = 0.0;
+        for (int k = 0; k < 9; k++) aa.gLc[((size_t)r * aa.nchunks + item) * 9 + k] = 0.0;
     if (tid == 0) {
-      aa.chunk_listed[chunk] = any_listed ? 1 : 0;
+      if (aa.run != 1) aa.chunk_listed[item] = any_listed ? 1 : 0;
       atomicAdd(a.count + MX_COUNT_QUEUE, end_cell - first_cell);
-      c.ints[1] = (int)(gridDim.x + atomicAdd(aa.chunk_queue, 1));
+      c.ints[1] = (int)(gridDim.x + atomicAdd(aa.run_queue, 1));
     }
     __syncthreads();
-    chunk = c.ints[1];
+    item = c.ints[1];
     __syncthreads();
   }
 }
@@ -1159,10 +1162,11 @@ __global__ void __launch_bounds__(32 * W, 3) vjp_recover_kernel(const Net net, c
           reverse_pass<W, R, true>(net, c, b, aa, sl, s0, n, dt, nd, pr, a.rtol, a.atol, sb, tid);
         }
         finish_cell(net, c, b, aa, sl, cell, Tc, P, nd, hin, dt, k, sb, failed, c.v, b.Nn, tid, nt);
-        // the cell's rate-table cotangent into its list slot, for the fixed-order sum
+        // the cell's rate-table cotangent into its slot, for the fixed-order sum
         const double* gl = adj_gl(net, aa, sl);
-        for (int e = tid; e < 3 * net.nr; e += nt) aa.gLq[(size_t)q * 3 * net.nr + e] = gl[e];
-        if (tid == 0) aa.pos[cell] = q;
+        const int at = aa.run == 1 ? cell : q;
+        for (int e = tid; e < 3 * net.nr; e += nt) aa.gLq[(size_t)at * 3 * net.nr + e] = gl[e];
+        if (tid == 0) aa.pos[cell] = at;
         __syncthreads();
         q = nq;
         break;
@@ -1171,8 +1175,52 @@ __global__ void __launch_bounds__(32 * W, 3) vjp_recover_kernel(const Net net, c
   }
 }
 
+// The chunks' partial sums from the cells' slots (run 1): add_to_chunk's operations in its order, one thread per
+// reaction. Block x: a chunk; y: SUMS_THREADS reactions. Reads each slot once, consecutive threads consecutive
+// addresses: bound by HBM (43 MB at 4,096 cells of 438 reactions).
+constexpr int SUMS_THREADS = 128;
+__global__ void __launch_bounds__(SUMS_THREADS) chunk_sums_kernel(const Net net, const CallArgs a, const AdjArgs aa) {
+  __shared__ double lT[ADJ_CHUNK], iT[ADJ_CHUNK];
+  __shared__ int passed[ADJ_CHUNK];
+  const int chunk = (int)blockIdx.x, tid = (int)threadIdx.x, r = (int)blockIdx.y * SUMS_THREADS + tid;
+  const int64_t c0 = (int64_t)chunk * ADJ_CHUNK;
+  const int n = (int)min((int64_t)ADJ_CHUNK, a.B - c0);
+  int listed = 0;
+  if (tid < n) {
+    const double Tc = a.T[c0 + tid];
+    lT[tid] = log(Tc);
+    iT[tid] = 1.0 / Tc;
+    const int flag = a.flag[c0 + tid];
+    listed = flag != 0;
+    passed[tid] = flag == 0 && a.status[c0 + tid] == 0;
+  }
+  listed = __syncthreads_or(listed);
+  if (blockIdx.y == 0 && tid == 0) aa.chunk_listed[chunk] = listed ? 1 : 0;
+  if (r >= net.nr) return;
+  double s[9];
+#pragma unroll
+  for (int j = 0; j < 9; j++) s[j] = 0.0;
+  bool first = true;
+#pragma unroll 4
+  for (int k = 0; k < n; k++) {
+    if (!passed[k]) continue;
+    const double* gl = aa.gLq + ((size_t)(c0 + k) * net.nr + r) * 3;
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+      const double g = gl[e];
+      s[3 * e] = first ? g : s[3 * e] + g;
+      s[3 * e + 1] = first ? g * lT[k] : fma(g, lT[k], s[3 * e + 1]);
+      s[3 * e + 2] = first ? -g * iT[k] : fma(-g, iT[k], s[3 * e + 2]);
+    }
+    first = false;
+  }
+  double* dst = aa.gLc + ((size_t)r * aa.nchunks + chunk) * 9;
+#pragma unroll
+  for (int j = 0; j < 9; j++) dst[j] = s[j];
+}
+
 // The rate table's cotangent: per reaction (one block; one thread per column), the chunks' partial sums in chunk order,
-// each chunk followed by its recovered cells in cell order (their list slots' cotangents times 1, ln T, -1 / T); cells
+// each chunk followed by its recovered cells in cell order (their slots' cotangents times 1, ln T, -1 / T); cells
 // that still fail (flag 2) or were refused are left out. Photolysis rows are 0. A fixed order: the same inputs give
 // the same bits, whatever the queues did. The block brings ARRH_TILE chunks at a time into shared memory (their 9
 // doubles are contiguous), so that the sums wait for an add and not for a load per chunk.
@@ -1194,7 +1242,7 @@ __global__ void __launch_bounds__(ARRH_THREADS) arrh_kernel(const Net net, const
         for (int k = 0; k < nk; k++) {
           acc += part[9 * k + j];
           if (!listed[k]) continue;
-          const int64_t c0 = (int64_t)(k0 + k) * aa.chunk, c1 = min((int64_t)a.B, c0 + aa.chunk);
+          const int64_t c0 = (int64_t)(k0 + k) * ADJ_CHUNK, c1 = min((int64_t)a.B, c0 + ADJ_CHUNK);
           for (int64_t cell = c0; cell < c1; cell++) {
             if (a.flag[cell] != 1) continue;  // passed (in the chunk's sum), still failed or refused
             const double g = aa.gLq[((size_t)aa.pos[cell] * net.nr + r) * 3 + e], Tc = a.T[cell];

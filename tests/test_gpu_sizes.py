@@ -71,3 +71,53 @@ def test_conversions_at_the_sizes_where_a_lanes_rows_change(gpu, species, cells)
     # positive sums of at most 254 terms in two orders (254 x 1.1e-16), a few roundings beside
     for got, exact in ((x.cpu().numpy(), ref), (back, want)):
         assert np.abs(got - exact).max() <= 6e-14 * exact.max() and (np.abs(got / exact - 1.0) <= 6e-14).all()
+
+
+def chunked(net, gpu, cells: int, **options):
+    """A solver, a batch and its cotangents for the tests of the rate table's sum."""
+    rng = np.random.default_rng(cells)
+    x = rng.uniform(0.1, 1.0, (cells, len(net.species)))
+    t = lambda a: torch.tensor(a, dtype=torch.float64, device=gpu)  # noqa: E731
+    args = [t(x / x.sum(1, keepdims=True)), t(rng.uniform(800.0, 1500.0, cells)), t(np.full(cells, 1e5)),
+            t(np.full(cells, 1e-6)), t(np.full(cells, 1e-9))]  # fmt: skip
+    return ADSolver(net, gpu, **options), args, t(rng.standard_normal(x.shape))
+
+
+# a cell a queue item up to 256 times the resident CTAs (113,664 or 151,552 cells), 64 above
+@pytest.mark.parametrize("cells", [64, 65, 1000, 4001, 60000, 200000])
+def test_the_rate_tables_cotangent_adds_fixed_chunks_of_64_cells_in_order(gpu, tmp_path, cells):
+    net, _ = invented.hydrogen(tmp_path)
+    solver, args, gx = chunked(net, gpu, cells)
+    chunks = -(-cells // 64)
+    used = range(chunks) if chunks <= 70 else [0, 1, chunks // 2, chunks - 2, chunks - 1]
+    keep = torch.zeros(cells, 1, dtype=torch.bool, device=gpu)
+    for k in used:
+        keep[64 * k : 64 * (k + 1)] = True
+    gx = torch.where(keep, gx, 0.0)  # the other chunks add zeros
+    with solver:
+        whole = solver.vjp(*args, gx).cotangents.rc
+        assert bool((solver.flag == 0).all()) and float(whole.abs().max()) > 0.0
+        total = torch.zeros_like(whole)
+        for k in used:
+            of = slice(64 * k, min(64 * (k + 1), cells))
+            total = total + solver.vjp(*(a[of].clone() for a in args), gx[of].clone()).cotangents.rc
+    assert torch.equal(whole, total)
+
+
+def test_recovered_cells_follow_their_chunk_in_the_rate_tables_sum(gpu, tmp_path):
+    net, _ = invented.hydrogen(tmp_path)
+    solver, args, gx = chunked(net, gpu, 150, drift=0.0)  # no drift allowed: many cells go through the recovery
+    with solver:
+        whole = solver.vjp(*args, gx).cotangents.rc[:, 0::3]  # the columns whose terms are the cells' own values
+        flag = solver.flag.tolist()
+        own = [solver.vjp(*(a[i : i + 1].clone() for a in args), gx[i : i + 1].clone()).cotangents.rc[:, 0::3]
+               for i in range(150)]  # fmt: skip
+    assert 0 in flag and 1 in flag
+    total = torch.zeros_like(whole)
+    for start in range(0, 150, 64):
+        cells = range(start, min(start + 64, 150))
+        passed = [own[i] for i in cells if flag[i] == 0]
+        total = total + sum(passed[1:], passed[0]) if passed else total
+        for i in cells:
+            total = total + own[i] if flag[i] == 1 else total
+    assert torch.equal(whole, total)
