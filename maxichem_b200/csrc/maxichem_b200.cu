@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <stdexcept>
 #include <vector>
 
 #include "solver.cuh"
@@ -642,7 +643,60 @@ __global__ void add_escalated_kernel(const int* sel_count, long long* escalated)
 // The place of round q's word of thread t with four consecutive rounds of a thread together, and the words of such a
 // stream: whole groups and a spare one, which a thread's reads ahead may touch.
 inline size_t grouped(int q, int t, int threads) { return ((size_t)(q / 4) * threads + t) * 4 + q % 4; }
-inline size_t grouped_words(int rounds, int threads) { return ((size_t)(rounds + 3) / 4 + 1) * threads * 4; }
+inline size_t grouped_words(int rounds, int threads) { return (((size_t)rounds + 3) / 4 + 1) * threads * 4; }
+
+// whether the words that mx_create regroups are there to be read
+bool streams_present(const mx_network* n) {
+  for (int g = 0; g < 2; g++) {
+    const int rounds[4] = {n->sv_rounds[g], n->sv_nrows[g], n->jac_rounds[g], n->jac_nents[g]};
+    const void* words[4] = {n->sv_stream[g], n->sv_rows[g], n->jac_stream[g], n->jac_dst[g]};
+    for (int q = 0; q < 4; q++)
+      if (rounds[q] < 0 || (rounds[q] > 0 && !words[q])) return false;
+  }
+  return true;
+}
+
+// The thread streams on the device, four words of a thread together; no host memory for them is the same error as no
+// device memory.
+cudaError_t upload_streams(mx_solver* s, const mx_network* n) try {
+  Net& net = s->net;
+  const int ns = net.ns, nr = net.nr;
+  cudaError_t e = cudaSuccess;
+  for (int g = 0; g < 2 && e == cudaSuccess; g++) {
+    const int t = n->stream_threads[g];
+    net.st_threads[g] = t;
+    net.sv_rounds[g] = n->sv_rounds[g];
+    // a thread's words with the piece that each one's end writes (sv_rows lists a thread's pieces in turn)
+    std::vector<uint32_t> w(grouped_words(n->sv_rounds[g], t), (uint32_t)nr);
+    for (int i = 0; i < t; i++)
+      for (int q = 0, k = 0; q < n->sv_rounds[g]; q++) {
+        const uint32_t word = n->sv_stream[g][(size_t)q * t + i];
+        const bool end = (word & 0x2000u) != 0 && k < n->sv_nrows[g];
+        w[grouped(q, i, t)] = word | (end ? (uint32_t)n->sv_rows[g][(size_t)k * t + i] << 16 : 0u);
+        k += end ? 1 : 0;
+      }
+    e = upload(s, (const uint4*)w.data(), w.size() / 4, &net.sv[g]);
+  }
+  {
+    const int t = n->stream_threads[0], rounds = n->jac_rounds[0];
+    net.jac_rounds = rounds;
+    std::vector<uint32_t> w(grouped_words(rounds, t), (uint32_t)(2 * nr) | (uint32_t)ns << 16 | (uint32_t)ns << 24);
+    std::vector<uint16_t> to(w.size(), 0);
+    for (int i = 0; i < t; i++)
+      for (int q = 0, k = 0; q < rounds; q++) {
+        const uint32_t word = n->jac_stream[0][(size_t)q * t + i];
+        w[grouped(q, i, t)] = word;
+        if ((word & 0x4000u) && k < n->jac_nents[0]) to[grouped(q, i, t)] = n->jac_dst[0][(size_t)k++ * t + i];
+      }
+    if (e == cudaSuccess) e = upload(s, (const uint4*)w.data(), w.size() / 4, &net.jt);
+    if (e == cudaSuccess) e = upload(s, (const uint2*)to.data(), to.size() / 4, &net.jd);
+  }
+  return e;
+} catch (const std::bad_alloc&) {
+  return cudaErrorMemoryAllocation;
+} catch (const std::length_error&) {
+  return cudaErrorMemoryAllocation;
+}
 
 }  // namespace
 
@@ -655,6 +709,10 @@ extern "C" int mx_create(const mx_network* n, double drift, int device, mx_solve
   if (n->ns < 1 || n->ns > MX_MAX_SPECIES || n->nr < 0 || n->nr >= 2048 || n->nel < 1 || n->nel > MX_MAX_ELEMENTS ||
       n->nj != n->nr - n->nrt || n->n_entries < 0) {
     set_error(err, errlen, "mx_create: network sizes out of range (ns %d, nr %d, nel %d)", n->ns, n->nr, n->nel);
+    return MX_ERR_NETWORK;
+  }
+  if (!streams_present(n)) {
+    set_error(err, errlen, "mx_create: a thread stream of a negative length or without its words");
     return MX_ERR_NETWORK;
   }
   if (!(drift >= 0.0 && drift <= 1e300)) {
@@ -759,35 +817,7 @@ extern "C" int mx_create(const mx_network* n, double drift, int device, mx_solve
   if (e == cudaSuccess) e = upload(s, n->jac_term, njt, &net.jac_term);
   net.n_pieces = n->n_pieces;
   if (e == cudaSuccess) e = upload(s, n->sv_row_ptr, ns + 1, &net.sv_row_ptr);
-  for (int g = 0; g < 2 && e == cudaSuccess; g++) {
-    const int t = n->stream_threads[g];
-    net.st_threads[g] = t;
-    net.sv_rounds[g] = n->sv_rounds[g];
-    // a thread's words with the piece that each one's end writes (sv_rows lists a thread's pieces in turn)
-    std::vector<uint32_t> w(grouped_words(n->sv_rounds[g], t), (uint32_t)nr);
-    for (int i = 0; i < t; i++)
-      for (int q = 0, k = 0; q < n->sv_rounds[g]; q++) {
-        const uint32_t word = n->sv_stream[g][(size_t)q * t + i];
-        const bool end = (word & 0x2000u) != 0 && k < n->sv_nrows[g];
-        w[grouped(q, i, t)] = word | (end ? (uint32_t)n->sv_rows[g][(size_t)k * t + i] << 16 : 0u);
-        k += end ? 1 : 0;
-      }
-    e = upload(s, (const uint4*)w.data(), w.size() / 4, &net.sv[g]);
-  }
-  {
-    const int t = n->stream_threads[0], rounds = n->jac_rounds[0];
-    net.jac_rounds = rounds;
-    std::vector<uint32_t> w(grouped_words(rounds, t), (uint32_t)(2 * nr) | (uint32_t)ns << 16 | (uint32_t)ns << 24);
-    std::vector<uint16_t> to(w.size(), 0);
-    for (int i = 0; i < t; i++)
-      for (int q = 0, k = 0; q < rounds; q++) {
-        const uint32_t word = n->jac_stream[0][(size_t)q * t + i];
-        w[grouped(q, i, t)] = word;
-        if ((word & 0x4000u) && k < n->jac_nents[0]) to[grouped(q, i, t)] = n->jac_dst[0][(size_t)k++ * t + i];
-      }
-    if (e == cudaSuccess) e = upload(s, (const uint4*)w.data(), w.size() / 4, &net.jt);
-    if (e == cudaSuccess) e = upload(s, (const uint2*)to.data(), to.size() / 4, &net.jd);
-  }
+  if (e == cudaSuccess) e = upload_streams(s, n);
   if (e != cudaSuccess) {
     set_error(err, errlen, "mx_create: %s", cudaGetErrorString(e));
     release(s);

@@ -46,6 +46,21 @@ def test_create_refuses_a_null_network_without_touching_a_device():
     assert b"null" in err.value
 
 
+@pytest.mark.parametrize("group", [0, 1])
+@pytest.mark.parametrize("field", ["sv_rounds", "sv_nrows", "jac_rounds", "jac_nents", "sv_stream", "sv_rows",
+                                   "jac_stream", "jac_dst"])  # fmt: skip
+def test_create_refuses_thread_streams_that_cannot_be_read(networks, field, group):
+    from maxichem_b200 import tables
+
+    s = abi.NetworkStruct(tables.build(networks("cho41"), True))
+    # a count below zero; words that are counted but not there
+    getattr(s.struct, field)[group] = -1 if field.endswith(("rounds", "nrows", "nents")) else None
+    handle = ctypes.c_void_p()
+    err = ctypes.create_string_buffer(256)
+    rc = abi.library().mx_create(s.ref(), 1e-6, 0, ctypes.byref(handle), err, 256)
+    assert rc == 3 and handle.value is None and b"stream" in err.value  # before any device is looked at
+
+
 def test_destroy_and_info_accept_null():
     lib = abi.library()
     assert lib.mx_destroy(None) == 0
