@@ -38,8 +38,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W) call_kernel(const Net net, con
     for (int q = 0; q < PH_COUNT; q++) ph[q] = 0;
     t0 = clock64();
   }
+  // every lane reads the clock: a branch for thread 0 here leaves warp 0 in two parts, whose shuffles and barriers of the
+  // solves that follow then run twice
   auto mark = [&](int q) {
-    if (PROF && tid == 0) {
+    if (PROF) {
       const long long t = clock64();
       ph[q] += t - t0;
       t0 = t;

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(32 * W, 20 / W)
     t0 = clock64();
   }
   auto mark = [&](int q) {
-    if (PROF && tid == 0) {
+    if (PROF) {
       const long long t = clock64();
       ph[q] += t - t0;
       t0 = t;
