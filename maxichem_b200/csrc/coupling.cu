@@ -1,12 +1,13 @@
 // The GCM step's conversions either side of a call (maxichem/coupling/composition.py:102-183 of the reference): mass
 // mixing ratios q [B][ns] to mole fractions x = (q / mw) / sum(q / mw), and back, q = x mw (mass / sum(x mw)). One
 // warp per cell streams its row (consecutive lanes, consecutive addresses), so each conversion reads and writes
-// [B][ns] once: the FP64 divisions and HBM share the time. Row sums are formed in the warp's order (lane l adds entries l, l + 32, ..., then a
-// butterfly). Problems are reported as bits or-ed into one word for the host to explain.
+// [B][ns] once: the FP64 divisions and HBM share the time. Row sums are formed in the warp's order (lane l adds entries
+// l, l + 32, ..., then a butterfly). Problems are reported as bits or-ed into one word for the host to explain.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 #include <cstdio>
+#include <type_traits>
 
 #include "../../include/maxichem_b200.h"
 
@@ -22,9 +23,11 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // q -> x. bad bits: 1 a non-finite q, 2 a negative q (unless signed_ok), 4 a cell whose sum of q / mw is not above 0.
-// A lane keeps its R quotients (species lane, lane + 32, ...; R by the species count: 2 to 64, 3 to 96, else 8) between the
-// sum and the result: the FP64 divisions, not the memory, were the time, three per value and now two, and the row's
-// loads are under way together. 262,144 cells of 69 species, both conversions with their host checks: 425 to 343 us.
+// A lane keeps its R = ceil(ns / 32) quotients (species lane, lane + 32, ...) between the sum and the result: the FP64
+// divisions, not the memory, were the time, three per value and now two, and the row's loads are under way together.
+// R is exact, since a row of padding alone costs its divisions too. Microseconds of 262,144 cells with a quotient
+// formed anew for each use, and so: 5 species 58 and 54, 69 species 150 and 105, 128 species 210 and 110, 254 species
+// 524 and 247 (with R 2, 3 or 8 only: 83, 106, 251 and 247).
 template <int R>
 __global__ void __launch_bounds__(32 * WARPS) mass_to_mole_kernel(const double* __restrict__ q,
                                                                   const double* __restrict__ mw, int64_t B, int ns,
@@ -105,6 +108,16 @@ int grid_for(int64_t B) {
   return (int)(blocks < most ? (blocks > 0 ? blocks : 1) : most);
 }
 
+// f with the row count r (1 .. MAX_ROWS) as a constant
+constexpr int MAX_ROWS = (MX_MAX_SPECIES + 31) / 32;
+template <int R = 1, class F>
+void for_rows(int r, const F& f) {
+  if (r == R)
+    f(std::integral_constant<int, R>{});
+  else if constexpr (R < MAX_ROWS)
+    for_rows<R + 1>(r, f);
+}
+
 }  // namespace
 
 extern "C" int mx_mass_to_mole(const double* q, const double* mw, int64_t B, int32_t ns, int32_t signed_ok,
@@ -113,13 +126,9 @@ extern "C" int mx_mass_to_mole(const double* q, const double* mw, int64_t B, int
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int32_t), st);
   if (e == cudaSuccess && B > 0) {
-    auto launch = [&](auto kernel) { kernel<<<grid_for(B), 32 * WARPS, 0, st>>>(q, mw, B, ns, signed_ok, x, bad); };
-    if (ns <= 64)
-      launch(mass_to_mole_kernel<2>);
-    else if (ns <= 96)
-      launch(mass_to_mole_kernel<3>);
-    else
-      launch(mass_to_mole_kernel<8>);
+    for_rows((ns + 31) / 32, [&](auto rows) {
+      mass_to_mole_kernel<decltype(rows)::value><<<grid_for(B), 32 * WARPS, 0, st>>>(q, mw, B, ns, signed_ok, x, bad);
+    });
     e = cudaGetLastError();
   }
   return e == cudaSuccess ? MX_OK : MX_ERR_CUDA;
@@ -131,13 +140,9 @@ extern "C" int mx_mole_to_mass(const double* x, const double* mw, const double* 
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int32_t), st);
   if (e == cudaSuccess && B > 0) {
-    auto launch = [&](auto kernel) { kernel<<<grid_for(B), 32 * WARPS, 0, st>>>(x, mw, mass, B, ns, q, bad); };
-    if (ns <= 64)
-      launch(mole_to_mass_kernel<2>);
-    else if (ns <= 96)
-      launch(mole_to_mass_kernel<3>);
-    else
-      launch(mole_to_mass_kernel<8>);
+    for_rows((ns + 31) / 32, [&](auto rows) {
+      mole_to_mass_kernel<decltype(rows)::value><<<grid_for(B), 32 * WARPS, 0, st>>>(x, mw, mass, B, ns, q, bad);
+    });
     e = cudaGetLastError();
   }
   return e == cudaSuccess ? MX_OK : MX_ERR_CUDA;

@@ -56,7 +56,7 @@ def test_the_rate_tables_cotangent_is_the_sum_over_the_cells(gpu, tmp_path, cell
 
 
 @pytest.mark.parametrize("cells", [1, 9, 9473])
-@pytest.mark.parametrize("species", [1, 31, 32, 33, 64, 65, 96, 97, 254])
+@pytest.mark.parametrize("species", [1, 31, 32, 33, 64, 65, 96, 97, 128, 129, 160, 161, 192, 193, 224, 225, 254])
 def test_conversions_at_the_sizes_where_a_lanes_rows_change(gpu, species, cells):
     rng = np.random.default_rng(species + cells)
     q, mw = 10.0 ** rng.uniform(-12.0, 0.0, (cells, species)), rng.uniform(1e-3, 1e-1, species)
