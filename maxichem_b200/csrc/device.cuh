@@ -48,6 +48,7 @@ struct Net {
   // residual (oR) and a stage's right side (oB); the plain layout leaves them 0.
   int ld, oA, oK, oV, on, oN, oY, oF, oU, oK1, oK2, oK3, oK4, oD, oRed, oInts, oPart, oG, doubles, a_doubles;
   int oS, oDg, onN, oW, oR, oB;
+  unsigned sms;  // of the device
 };
 
 struct CallArgs {
@@ -99,12 +100,12 @@ __device__ __forceinline__ Cell cell_arrays(const Net& net, double* smem) {
 // solves, so the warps 0 of an SM's CTAs should sit on different schedulers. The device gives 4-warp CTAs' warps slots
 // that do (measured: 0 1 2 3, 5 6 7 4, 10 11 8 9, 15 12 13 14; rotating them here put all four on one scheduler, 98
 // against 84 ms for 65,536 cells of 69 species), 2-warp CTAs' ones slots 0 1, 2 3, 4 5, ..., two schedulers of four
-// (39.6 against 38.6 ms for 40,000 cells of 41 species).
+// (a settled call of 40,000 cells of 41 species: 9.77 ms without the exchange, 9.31 with it; 1,000 cells 0.48 and 0.47).
+// It takes CTA b for the (b / SMs)-th of its SM, the order in which a grid's first CTAs were dealt out here; where a
+// device deals them out otherwise, results are the same and the exchange may gain nothing.
 template <int W>
-__device__ __forceinline__ int spread_tid() {
+__device__ __forceinline__ int spread_tid(unsigned sms) {
   if (W != 2) return (int)threadIdx.x;
-  unsigned sms;
-  asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
   const int turn = (int)(blockIdx.x / sms) / 2;
   return (int)((threadIdx.x + 32 * turn) % (32 * W));
 }

@@ -31,7 +31,7 @@ template <int W, int R, bool PROF, bool LIST = false>
 __global__ void __launch_bounds__(32 * W, 16 / W) call_kernel(const Net net, const CallArgs a, long long* prof) {
   extern __shared__ double smem[];
   const Cell c = cell_arrays(net, smem);
-  const int tid = spread_tid<W>(), nt = 32 * W, lane = tid & 31, warp = tid >> 5, ns = net.ns, ld = net.ld;
+  const int tid = spread_tid<W>(net.sms), nt = 32 * W, lane = tid & 31, warp = tid >> 5, ns = net.ns, ld = net.ld;
   long long ph[PH_COUNT], t0 = 0;
   if (PROF) {
 #pragma unroll
@@ -758,6 +758,7 @@ extern "C" int mx_create(const mx_network* n, double drift, int device, mx_solve
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
   cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, device);
+  net.sms = (unsigned)s->sms;
   if ((size_t)optin < s->smem) {
     set_error(err, errlen, "one cell needs %zu B of shared memory; the device has %d per block", s->smem, optin);
     delete s;
