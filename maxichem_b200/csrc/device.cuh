@@ -19,7 +19,6 @@ constexpr double RODAS_C43 = 8.0 / 3.0;  // stage coupling, -C_43
 constexpr double TROE_C0 = 0.4, TROE_C1 = 0.67, TROE_N0 = 0.75, TROE_N1 = 1.27, TROE_D = 0.14;  // Venot et al. 2012
 constexpr int FL_FALLOFF = 1, FL_SECOND_K0 = 2, FL_THREE_BODY = 4, FL_TROE = 64, FL_EFF = 128, FL_VM11 = 512;
 constexpr int GUARD_NONFINITE = 4, GUARD_UNFINISHED = 8, GUARD_DRIFT = 16;
-constexpr int PANEL = 8;  // pivots per block of the blocked LU
 
 // A network's tables on the device, and the per-CTA shared-memory layout (offsets in doubles).
 struct Net {
@@ -359,156 +358,21 @@ __device__ __forceinline__ void jacobian_w(const Net& net, const Cell& c, double
   __syncthreads();
 }
 
-// ---- dense LU without exchanges, blocked (PANEL pivots at a time), with a lookahead of one panel: the mixed path's
-// FP32 factors (the FP64 ones are lu_mma's) ----
+// ---- the LU without exchanges, on the matrix pipe ----
 // Every entry receives its updates A_ij <- fma(-l_ik, A_kj, A_ij) in ascending k, l_ik = A_ik / A_kk taken as
 // A_ik * (1 / A_kk): the order and the operations of the right-looking LU, so the bits of the sparse factorisation
-// on the fill pattern (call.cuh:81-112) for finite data. Per block: the block's pivot rows beyond the panel (one
-// thread per column); then warp 0 applies the block to the next panel's columns and factors that panel (one lane per
-// row, warp syncs only) while warps 1-3 apply it to the columns past the next panel, as a rank-PANEL update in 4 x 4
-// register tiles (rows and columns cyclic, so a warp's loads are broadcast or consecutive).
-
-// the element type's correctly rounded reciprocal (FP64 for the plain path, FP32 for the mixed path's factors)
-__device__ __forceinline__ double rcp_rn(double a) { return __drcp_rn(a); }
-__device__ __forceinline__ float rcp_rn(float a) { return __frcp_rn(a); }
-
-// the trailing update of rows ke.. and columns cs.. (cs >= ke) by NT threads
-template <int NT, typename T>
-__device__ __forceinline__ void trailing_update_from(T* A, int ld, int kb, int nb, int ke, int cs, int ns, int tid) {
-  constexpr int CG = 16, RG = NT / CG;
-  const int cg = tid % CG, rg = tid / CG, m = ns - ke, mc = ns - cs;
-  for (int rb = rg; rb < m; rb += 4 * RG) {
-    for (int cb = cg; cb < mc; cb += 4 * CG) {
-      int row[4], col[4];
-      bool rok[4], cok[4];
-#pragma unroll
-      for (int a = 0; a < 4; a++) {
-        rok[a] = rb + RG * a < m;
-        row[a] = ke + (rok[a] ? rb + RG * a : 0);
-        cok[a] = cb + CG * a < mc;
-        col[a] = cs + (cok[a] ? cb + CG * a : 0);
-      }
-      T acc[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = A[row[a] * ld + col[b]];
-#pragma unroll 2
-      for (int t = 0; t < PANEL; t++) {
-        if (t < nb) {
-          T l[4], u[4];
-#pragma unroll
-          for (int a = 0; a < 4; a++) {
-            l[a] = A[row[a] * ld + kb + t];
-            u[a] = A[(kb + t) * ld + col[a]];
-          }
-#pragma unroll
-          for (int a = 0; a < 4; a++)
-#pragma unroll
-            for (int b = 0; b < 4; b++) acc[a][b] = fma(-l[a], u[b], acc[a][b]);
-        }
-      }
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-          if (rok[a] && cok[b]) A[row[a] * ld + col[b]] = acc[a][b];
-    }
-  }
-}
-
-// the panel kb .. kb + nb - 1 on one warp (lane), warp-level syncs only
-template <typename T>
-__device__ __forceinline__ void panel_warp(T* A, int ld, T* dinv, int kb, int nb, int ns, int lane) {
-  const int ke = kb + nb;
-  if (lane == 0) dinv[kb] = rcp_rn(A[kb * ld + kb]);
-  __syncwarp();
-  for (int k = kb; k < ke; k++) {
-    const T d = dinv[k];
-    T piv[PANEL];
-#pragma unroll
-    for (int jj = 1; jj < PANEL; jj++) piv[jj] = k + jj < ke ? A[k * ld + k + jj] : T(0);
-#pragma unroll 1
-    for (int i = k + 1 + lane; i < ns; i += 32) {
-      T* ai = A + i * ld;
-      const T l = ai[k] * d;
-      ai[k] = l;
-#pragma unroll
-      for (int jj = 1; jj < PANEL; jj++)
-        if (k + jj < ke) ai[k + jj] = fma(-l, piv[jj], ai[k + jj]);
-    }
-    // the next pivot is final now and its row is lane 0's (its first row), so lane 0 takes the reciprocal of its own
-    // write, after the row loop
-    if (lane == 0 && k + 1 < ke) dinv[k + 1] = rcp_rn(A[(k + 1) * ld + k + 1]);
-    __syncwarp();
-  }
-}
-
-// the blocked LU with a lookahead of one panel: while warps 1-3 apply panel p to the columns past panel p + 1, warp 0
-// applies it to panel p + 1's columns and factors panel p + 1. Each entry takes its updates in ascending pivot order.
-template <int NT, typename T>
-__device__ __forceinline__ void lu_factor(const Net& net, T* A, T* dinv, int tid) {
-  const int ns = net.ns, ld = net.ld, warp = tid >> 5, lane = tid & 31;
-  if (warp == 0) panel_warp(A, ld, dinv, 0, min(PANEL, ns), ns, lane);
-  __syncthreads();
-  for (int kb = 0; kb < ns; kb += PANEL) {
-    const int ke = min(kb + PANEL, ns), nb = ke - kb;
-    if (ke == ns) break;
-    for (int j = ke + tid; j < ns; j += NT) {  // the block's pivot rows beyond the panel
-      T row[PANEL];
-#pragma unroll
-      for (int s = 0; s < PANEL; s++) row[s] = s < nb ? A[(kb + s) * ld + j] : T(0);
-#pragma unroll
-      for (int s = 1; s < PANEL; s++) {
-        if (s < nb) {
-          T a = row[s];
-#pragma unroll
-          for (int t = 0; t < PANEL; t++)
-            if (t < s) a = fma(-A[(kb + s) * ld + kb + t], row[t], a);
-          row[s] = a;
-          A[(kb + s) * ld + j] = a;
-        }
-      }
-    }
-    __syncthreads();
-    const int ken = min(ke + PANEL, ns);
-    if (warp == 0) {
-#pragma unroll 1
-      for (int i = ke + lane; i < ns; i += 32) {  // panel p + 1's columns, rows ke..
-        T* ai = A + i * ld;
-        T l[PANEL];
-#pragma unroll
-        for (int t = 0; t < PANEL; t++) l[t] = t < nb ? ai[kb + t] : T(0);
-        for (int j = ke; j < ken; j++) {
-          T acc = ai[j];
-#pragma unroll
-          for (int t = 0; t < PANEL; t++)
-            if (t < nb) acc = fma(-l[t], A[(kb + t) * ld + j], acc);
-          ai[j] = acc;
-        }
-      }
-      __syncwarp();
-      panel_warp(A, ld, dinv, ke, ken - ke, ns, lane);
-    } else {
-      trailing_update_from<NT - 32, T>(A, ld, kb, nb, ke, ken, ns, tid - 32);
-    }
-    __syncthreads();
-  }
-}
-
-// ---- the FP64 LU on the matrix pipe ----
-// The same factorisation as lu_factor's (the same operations on every entry in ascending pivot order, so the same
-// bits), blocked by 8 with the trailing update as FP64 matrix instructions. mma.m8n8k4 adds its four products to an
-// entry one after the other in ascending k, each a correctly rounded fma: measured equal to the fma chain on 786,432
-// random entries over 24 binary orders of magnitude, at the FP64 pipe's full rate (36.8 TFLOP/s). One instruction does the work of
-// 8 warp-wide fma's, and an 8 x 8 tile needs 8 shared accesses a lane for 512 fma's.
+// on the fill pattern (call.cuh:81-112) for finite data. Blocked by 8, with the trailing update as FP64 matrix
+// instructions. mma.m8n8k4 adds its four products to an entry one after the other in ascending k, each a correctly
+// rounded fma: measured equal to the fma chain on 786,432 random entries over 24 binary orders of magnitude, at the
+// FP64 pipe's full rate (36.8 TFLOP/s). One instruction does the work of 8 warp-wide fma's, and an 8 x 8 tile needs 8
+// shared accesses a lane for 512 fma's.
 // Per block: the rows below it (L) on half of the warps and the columns right of it (U) on the other half, one lane
 // each, in registers; then warp 0 updates and factors the next diagonal block while the other warps update the rest.
-// What bounds it now is the chain of the diagonal blocks (69 pivots of a reciprocal, a product, an fma and a shuffle)
-// and shared-memory bandwidth: 69 species, one cell an SM, 25,000 cycles against lu_factor's 60,000, four cells an SM
-// 30,500 against 76,500. The loops are kept rolled where they can be: the whole try is 60 KB of code, and unrolled
-// forms that are faster alone (the diagonal block's pivots, 8-pivot solves) made the call 13 % slower with four cells
-// an SM, by instruction fetch.
+// What bounds it is the chain of the diagonal blocks (69 pivots of a reciprocal, a product, an fma and a shuffle) and
+// shared-memory bandwidth: 69 species, 26,300 cycles with one cell an SM, 39,900 with four that all factor at once (a
+// factorisation in 4 x 4 register tiles 60,000 and 76,500). The loops are kept rolled where they can be: the whole try is 60 KB of code,
+// and unrolled forms that are faster alone (the diagonal block's pivots, 8-pivot solves) made the call 13 % slower with
+// four cells an SM, by instruction fetch.
 
 // c (8 x 8: lane 4 g + t holds row g, columns 2 t and 2 t + 1) += a (8 x 4: row g, column t) b (4 x 8: row t, column g)
 __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
@@ -536,7 +400,7 @@ __device__ __forceinline__ void lu_diagonal(double& x0, double& x1, double* dinv
     const double below = __shfl_sync(FULL, a, 4 * k + 4 + q), right = __shfl_sync(FULL, b, 4 * k + n);
     const double next = __shfl_sync(FULL, b, 4 * k + 4 + n), col = __shfl_sync(FULL, a, 4 * g + q);
     const double u0 = __shfl_sync(FULL, x0, 4 * k + t), u1 = __shfl_sync(FULL, x1, 4 * k + t);
-    const double d = rcp_rn(piv);
+    const double d = __drcp_rn(piv);
     piv = fma(-(below * d), right, next);
     const double l = col * d, m = g > k ? l : 0.0;
     x0 = fma(-m, t > q ? u0 : 0.0, x0);
@@ -683,88 +547,30 @@ __device__ __forceinline__ double pick(const double (&a)[R], int idx) {
   return v;
 }
 
-// The forward and backward sweeps of M0^-1 on NV register-held vectors (a: lane l holds rows l + 32 p; d: 1 / U_kk),
-// the body of the mixed path's FP32 solve. On return a[v][p] * d[p] is the solution.
-template <int R, int NV, typename T>
-__device__ __forceinline__ void lu_sweep(const Net& net, const T* A, T (&a)[NV][R], const T (&d)[R], int lane) {
-  const int ns = net.ns, ld = net.ld, last = ns - 1;
-#pragma unroll
-  for (int c = 0; c < R; c++) {  // forward: pivots 32c .. 32c + 31
-    const int k0 = 32 * c, k1 = min(k0 + 32, last);
-    if (k0 >= k1) break;
-    T m[R];
-#pragma unroll
-    for (int p = c; p < R; p++) m[p] = A[min(lane + 32 * p, last) * ld + k0];
-#pragma unroll 2
-    for (int k = k0; k < k1; k++) {
-      T yk[NV];
-#pragma unroll
-      for (int v = 0; v < NV; v++) yk[v] = __shfl_sync(FULL, a[v][c], k & 31);
-      T mn[R];
-#pragma unroll
-      for (int p = c; p < R; p++) mn[p] = A[min(lane + 32 * p, last) * ld + min(k + 1, last)];
-#pragma unroll
-      for (int p = c; p < R; p++) {
-        const bool act = (p > c ? true : lane > k - k0) && lane + 32 * p < ns;
-        const T mm = act ? m[p] : T(0);
-#pragma unroll
-        for (int v = 0; v < NV; v++) a[v][p] = fma(-mm, yk[v], a[v][p]);
-        m[p] = mn[p];
-      }
-    }
-  }
-#pragma unroll
-  for (int c = R - 1; c >= 0; c--) {  // backward: pivots 32c + 31 .. 32c (down to 1)
-    const int k0 = 32 * c, khi = min(k0 + 31, last), klo = max(k0, 1);
-    if (khi < klo) continue;
-    T m[R];
-#pragma unroll
-    for (int p = 0; p <= c; p++) m[p] = A[min(lane + 32 * p, last) * ld + khi];
-#pragma unroll 2
-    for (int k = khi; k >= klo; k--) {
-      T z[NV];
-#pragma unroll
-      for (int v = 0; v < NV; v++) z[v] = __shfl_sync(FULL, a[v][c] * d[c], k & 31);
-      T mn[R];
-#pragma unroll
-      for (int p = 0; p <= c; p++) mn[p] = A[min(lane + 32 * p, last) * ld + max(k - 1, 0)];
-#pragma unroll
-      for (int p = 0; p <= c; p++) {
-        const bool act = p < c ? true : lane < k - k0;
-        const T mm = act ? m[p] : T(0);
-#pragma unroll
-        for (int v = 0; v < NV; v++) a[v][p] = fma(-mm, z[v], a[v][p]);
-        m[p] = mn[p];
-      }
-    }
-  }
-}
-
-// y <- M0^-1 y on one warp for NV vectors (1 or 2) with the factors of the LU: lane l holds rows l + 32 p. Forward unit
+// y <- M0^-1 y on one warp with the factors of the LU: lane l holds rows l + 32 p. Forward unit
 // L in ascending k, U in descending k with x_k = a_k / U_kk (msolve, common.cuh:504-522). Each entry receives the
 // one-pivot sweep's fma's in its order, four pivots at a time: their four values are gathered from their lanes, every
 // lane solves the 4 x 4 block alike (its entries are broadcast reads) and applies the four to its rows, so four
 // pivots cost one shuffle latency instead of four; the matrix's last rows past a multiple of four go one by one. One
 // warp issues it, so its instructions and their latencies are the time: 8,500 cycles at 69 species.
 // Not inlined: the call kernel solves at four places, and one copy of the code keeps the instruction cache warm; the
-// vectors and the matrix are offsets into shared memory, so that its accesses stay shared ones.
-// With oU >= 0 the Sherman-Morrison correction of W = M0 - w 1^T follows on the first vector (sherman's operations).
-template <int R, int NV>
-__device__ __noinline__ void lu_solve_at(int ns, int ld, int oA, int oD, int o0, int o1, int oU, double c0, int lane) {
+// vector and the matrix are offsets into shared memory, so that its accesses stay shared ones.
+// With oU >= 0 the Sherman-Morrison correction of W = M0 - w 1^T follows (sherman's operations).
+template <int R>
+__device__ __noinline__ void lu_solve_at(int ns, int ld, int oA, int oD, int oY, int oU, double c0, int lane) {
   extern __shared__ double smem[];
   const double* A = smem + oA;
   const double* dinv = smem + oD;
-  double* y[2] = {smem + o0, smem + o1};
+  double* y = smem + oY;
   const int last = ns - 1, tail = ns & ~3;  // pivots tail .. last one by one
-  double a[NV][R], d[R];
+  double a[R], d[R];
   const double* row[R];
 #pragma unroll
   for (int p = 0; p < R; p++) {
     const int i = min(lane + 32 * p, last);
     row[p] = A + i * ld;
     d[p] = dinv[i];
-#pragma unroll
-    for (int v = 0; v < NV; v++) a[v][p] = y[v][i];
+    a[p] = y[i];
   }
   const double* dg = A;  // the block's diagonal
 #pragma unroll
@@ -775,39 +581,31 @@ __device__ __noinline__ void lu_solve_at(int ns, int ld, int oA, int oD, int o0,
       const int k = 32 * c + b;
       const double *d1 = dg + ld, *d2 = d1 + ld, *d3 = d2 + ld;
       const double l10 = d1[0], l20 = d2[0], l21 = d2[1], l30 = d3[0], l31 = d3[1], l32 = d3[2];
-      double l[R][4], g[NV][4];
+      double l[R][4], g[4];
 #pragma unroll
-      for (int v = 0; v < NV; v++)
-#pragma unroll
-        for (int s = 0; s < 4; s++) g[v][s] = __shfl_sync(FULL, a[v][c], b + s);
+      for (int s = 0; s < 4; s++) g[s] = __shfl_sync(FULL, a[c], b + s);
 #pragma unroll
       for (int p = c; p < R; p++)
 #pragma unroll
         for (int s = 0; s < 4; s++) l[p][s] = row[p][k + s];
+      g[1] = fma(-l10, g[0], g[1]);
+      g[2] = fma(-l20, g[0], g[2]);
+      g[3] = fma(-l30, g[0], g[3]);
+      g[2] = fma(-l21, g[1], g[2]);
+      g[3] = fma(-l31, g[1], g[3]);
+      g[3] = fma(-l32, g[2], g[3]);
 #pragma unroll
-      for (int v = 0; v < NV; v++) {
-        g[v][1] = fma(-l10, g[v][0], g[v][1]);
-        g[v][2] = fma(-l20, g[v][0], g[v][2]);
-        g[v][3] = fma(-l30, g[v][0], g[v][3]);
-        g[v][2] = fma(-l21, g[v][1], g[v][2]);
-        g[v][3] = fma(-l31, g[v][1], g[v][3]);
-        g[v][3] = fma(-l32, g[v][2], g[v][3]);
+      for (int s = 0; s < 4; s++)
 #pragma unroll
-        for (int s = 0; s < 4; s++)
-#pragma unroll
-          for (int p = c; p < R; p++)
-            if (p > c || lane > b + s) a[v][p] = fma(-l[p][s], g[v][s], a[v][p]);
-      }
+        for (int p = c; p < R; p++)
+          if (p > c || lane > b + s) a[p] = fma(-l[p][s], g[s], a[p]);
       dg = d3 + ld + 4;
     }
     if (R <= 4 ? c == R - 1 : c == last >> 5) {
 #pragma unroll 1
       for (int k = tail; k < last; k++) {
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-          const double yk = __shfl_sync(FULL, a[v][c], k & 31);
-          if (lane > (k & 31)) a[v][c] = fma(-row[c][k], yk, a[v][c]);
-        }
+        const double yk = __shfl_sync(FULL, a[c], k & 31);
+        if (lane > (k & 31)) a[c] = fma(-row[c][k], yk, a[c]);
       }
     }
   }
@@ -816,13 +614,10 @@ __device__ __noinline__ void lu_solve_at(int ns, int ld, int oA, int oD, int o0,
     if (R <= 4 ? c == R - 1 : c == last >> 5) {
 #pragma unroll 1
       for (int k = last; k >= tail; k--) {
+        const double z = __shfl_sync(FULL, a[c] * d[c], k & 31);
 #pragma unroll
-        for (int v = 0; v < NV; v++) {
-          const double z = __shfl_sync(FULL, a[v][c] * d[c], k & 31);
-#pragma unroll
-          for (int p = 0; p <= c; p++)
-            if (p < c || lane < (k & 31)) a[v][p] = fma(-row[p][k], z, a[v][p]);
-        }
+        for (int p = 0; p <= c; p++)
+          if (p < c || lane < (k & 31)) a[p] = fma(-row[p][k], z, a[p]);
       }
     }
     const int nb = min(32, tail - 32 * c);
@@ -833,59 +628,48 @@ __device__ __noinline__ void lu_solve_at(int ns, int ld, int oA, int oD, int o0,
       const double *e1 = dg + ld, *e2 = e1 + ld;
       const double u01 = dg[1], u02 = dg[2], u03 = dg[3], u12 = e1[2], u13 = e1[3], u23 = e2[3];
       const double d0 = dinv[k], d1 = dinv[k + 1], d2 = dinv[k + 2], d3 = dinv[k + 3];
-      double u[R][4], g[NV][4];
+      double u[R][4], g[4];
 #pragma unroll
-      for (int v = 0; v < NV; v++)
-#pragma unroll
-        for (int s = 0; s < 4; s++) g[v][s] = __shfl_sync(FULL, a[v][c], b + s);
+      for (int s = 0; s < 4; s++) g[s] = __shfl_sync(FULL, a[c], b + s);
 #pragma unroll
       for (int p = 0; p <= c; p++)
 #pragma unroll
         for (int s = 0; s < 4; s++) u[p][s] = row[p][k + s];
+      double z[4];
+      z[3] = g[3] * d3;
+      z[2] = fma(-u23, z[3], g[2]) * d2;
+      z[1] = fma(-u12, z[2], fma(-u13, z[3], g[1])) * d1;
+      z[0] = fma(-u01, z[1], fma(-u02, z[2], fma(-u03, z[3], g[0]))) * d0;
 #pragma unroll
-      for (int v = 0; v < NV; v++) {
-        double z[4];
-        z[3] = g[v][3] * d3;
-        z[2] = fma(-u23, z[3], g[v][2]) * d2;
-        z[1] = fma(-u12, z[2], fma(-u13, z[3], g[v][1])) * d1;
-        z[0] = fma(-u01, z[1], fma(-u02, z[2], fma(-u03, z[3], g[v][0]))) * d0;
+      for (int s = 3; s >= 0; s--)
 #pragma unroll
-        for (int s = 3; s >= 0; s--)
-#pragma unroll
-          for (int p = 0; p <= c; p++)
-            if (p < c || lane < b + s) a[v][p] = fma(-u[p][s], z[s], a[v][p]);
-      }
+        for (int p = 0; p <= c; p++)
+          if (p < c || lane < b + s) a[p] = fma(-u[p][s], z[s], a[p]);
     }
   }
 #pragma unroll
-  for (int v = 0; v < NV; v++)
-#pragma unroll
-    for (int p = 0; p < R; p++) a[v][p] *= d[p];
+  for (int p = 0; p < R; p++) a[p] *= d[p];
   if (oU >= 0) {
     const double* u = smem + oU;
     double s = 0.0;
 #pragma unroll
     for (int p = 0; p < R; p++)
-      if (lane + 32 * p < ns) s += a[0][p];
+      if (lane + 32 * p < ns) s += a[p];
     s = warp_sum(s) * c0;
 #pragma unroll
-    for (int p = 0; p < R; p++) a[0][p] = fma(s, u[min(lane + 32 * p, last)], a[0][p]);
+    for (int p = 0; p < R; p++) a[p] = fma(s, u[min(lane + 32 * p, last)], a[p]);
   }
   __syncwarp();
 #pragma unroll
-  for (int v = 0; v < NV; v++)
-#pragma unroll
-    for (int p = 0; p < R; p++)
-      if (lane + 32 * p < ns) y[v][lane + 32 * p] = a[v][p];
+  for (int p = 0; p < R; p++)
+    if (lane + 32 * p < ns) y[lane + 32 * p] = a[p];
   __syncwarp();
 }
 
-template <int R, int NV>
-__device__ __forceinline__ void lu_solve(const Net& net, const double* A, const double* dinv, double* y0, double* y1,
-                                         int lane) {
+template <int R>
+__device__ __forceinline__ void lu_solve(const Net& net, const double* A, const double* dinv, double* y, int lane) {
   extern __shared__ double smem[];
-  const int o0 = (int)(y0 - smem), o1 = NV == 2 ? (int)(y1 - smem) : o0;
-  lu_solve_at<R, NV>(net.ns, net.ld, (int)(A - smem), (int)(dinv - smem), o0, o1, -1, 0.0, lane);
+  lu_solve_at<R>(net.ns, net.ld, (int)(A - smem), (int)(dinv - smem), (int)(y - smem), -1, 0.0, lane);
 }
 
 // y <- W^-1 y on one warp: the solve and the Sherman-Morrison correction with u = M0^-1 w and c0 = 1 / (1 - sum u)
@@ -893,8 +677,7 @@ template <int R>
 __device__ __forceinline__ void w_solve(const Net& net, const double* A, const double* dinv, double* y, const double* u,
                                         double c0, int lane) {
   extern __shared__ double smem[];
-  const int o = (int)(y - smem);
-  lu_solve_at<R, 1>(net.ns, net.ld, (int)(A - smem), (int)(dinv - smem), o, o, (int)(u - smem), c0, lane);
+  lu_solve_at<R>(net.ns, net.ld, (int)(A - smem), (int)(dinv - smem), (int)(y - smem), (int)(u - smem), c0, lane);
 }
 
 // y <- y + c0 (sum y) u on one warp (sherman_morrison_update, common.cuh:542-557)
@@ -1044,7 +827,7 @@ __device__ __noinline__ void dense_lu_at(int ns, int ld, int oA, int oD, int oP,
           }
           __syncwarp();
         }
-        const double d = rcp_rn(u[0]);
+        const double d = __drcp_rn(u[0]);
 #pragma unroll
         for (int p = 0; p < R; p++) {
           const int i = lane + 32 * p;
@@ -1119,7 +902,7 @@ __device__ __forceinline__ void dense_solve(const Net& net, const double* A, con
   for (int p = 0; p < R; p++)
     if (lane + 32 * p < net.ns) y[lane + 32 * p] = a[p];
   __syncwarp();
-  lu_solve<R, 1>(net, A, dinv, y, nullptr, lane);
+  lu_solve<R>(net, A, dinv, y, lane);
 }
 
 // ---- step control (common.cuh:90-133) ----

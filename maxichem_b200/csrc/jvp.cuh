@@ -344,7 +344,7 @@ __device__ __forceinline__ void stage_solve(const Net& net, const Cell& c, doubl
   if (DENSE) {
     dense_solve<R>(net, c.A, c.dinv, pr, y, lane);
   } else {
-    lu_solve<R, 1>(net, c.A, c.dinv, y, nullptr, lane);
+    lu_solve<R>(net, c.A, c.dinv, y, lane);
     sherman(net, y, c.U, c0, lane);
   }
 }
@@ -676,9 +676,9 @@ __global__ void __launch_bounds__(32 * W, 3) jvp_kernel(const Net net, const Cal
       if (warp == 0) {
         for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
         __syncwarp();
-        lu_solve<R, 1>(net, c.A, c.dinv, c.K1, nullptr, lane);
+        lu_solve<R>(net, c.A, c.dinv, c.K1, lane);
       } else if (warp == 1) {
-        lu_solve<R, 1>(net, c.A, c.dinv, c.U, nullptr, lane);
+        lu_solve<R>(net, c.A, c.dinv, c.U, lane);
       }
       __syncthreads();
       if (warp == 0) {
@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(32 * W, 3) jvp_kernel(const Net net, const Cal
       }
       __syncthreads();
       if (warp == 0) {
-        lu_solve<R, 1>(net, c.A, c.dinv, c.K2, nullptr, lane);
+        lu_solve<R>(net, c.A, c.dinv, c.K2, lane);
         sherman(net, c.K2, c.U, c0, lane);
       } else {
         rhs(net, c, c.Y, false, nd, tid - 32, nt - 32, 1);
@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(32 * W, 3) jvp_kernel(const Net net, const Cal
       if (warp == 0) {
         for (int i = lane; i < ns; i += 32) c.K3[i] = fma(ih, c.K1[i] - c.K2[i], c.F[i]);
         __syncwarp();
-        lu_solve<R, 1>(net, c.A, c.dinv, c.K3, nullptr, lane);
+        lu_solve<R>(net, c.A, c.dinv, c.K3, lane);
         sherman(net, c.K3, c.U, c0, lane);
         for (int i = lane; i < ns; i += 32) c.Y[i] = c.N[i] + 2.0 * c.K1[i] + c.K3[i];
       }
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(32 * W, 3) jvp_kernel(const Net net, const Cal
         for (int i = lane; i < ns; i += 32)
           c.K4[i] = fma(ih, fma(-RODAS_C43, c.K3[i], c.K1[i] - c.K2[i]), c.F[i]);
         __syncwarp();
-        lu_solve<R, 1>(net, c.A, c.dinv, c.K4, nullptr, lane);
+        lu_solve<R>(net, c.A, c.dinv, c.K4, lane);
         sherman(net, c.K4, c.U, c0, lane);
         try_error<R>(net, c, s.t == 0.0, a.rtol, a.atol, lane);
       }

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(32 * W, 16 / W) call_kernel(const Net net, con
               for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
               __syncwarp();
             }
-            lu_solve<R, 1>(net, c.A, c.dinv, y, nullptr, lane);
+            lu_solve<R>(net, c.A, c.dinv, y, lane);
           }
           __syncthreads();
           if (warp == 0) {  // Sherman-Morrison, then stage 2's right side and Y3 = N + 2 K1
@@ -398,16 +398,20 @@ __global__ void __launch_bounds__(32 * W) debug_try_kernel(const Net net, const 
   for (int i = tid; i < ns; i += nt) o[i] = c.dinv[i];
   o += ns;
   double c0 = 0.0;
+  if (warp < 2) {  // K1 on warp 0 and M0^-1 w on warp 1
+    if (warp == 0) {
+      for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
+      __syncwarp();
+    }
+    lu_solve<R>(net, c.A, c.dinv, warp == 0 ? c.K1 : c.U, lane);
+  }
+  __syncthreads();
   if (warp == 0) {
-    for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
-    __syncwarp();
-    lu_solve<R, 2>(net, c.A, c.dinv, c.K1, c.U, lane);
     c0 = 1.0 / (1.0 - lane_sum(c.U, ns, lane));
     sherman(net, c.K1, c.U, c0, lane);
     for (int i = lane; i < ns; i += 32) c.K2[i] = fma(RODAS_C21 * ih, c.K1[i], c.F[i]);
     __syncwarp();
-    lu_solve<R, 1>(net, c.A, c.dinv, c.K2, nullptr, lane);
-    sherman(net, c.K2, c.U, c0, lane);
+    w_solve<R>(net, c.A, c.dinv, c.K2, c.U, c0, lane);
     for (int i = lane; i < ns; i += 32) c.Y[i] = c.N[i] + 2.0 * c.K1[i];
   }
   __syncthreads();
@@ -415,8 +419,7 @@ __global__ void __launch_bounds__(32 * W) debug_try_kernel(const Net net, const 
   if (warp == 0) {
     for (int i = lane; i < ns; i += 32) c.K3[i] = fma(ih, c.K1[i] - c.K2[i], c.F[i]);
     __syncwarp();
-    lu_solve<R, 1>(net, c.A, c.dinv, c.K3, nullptr, lane);
-    sherman(net, c.K3, c.U, c0, lane);
+    w_solve<R>(net, c.A, c.dinv, c.K3, c.U, c0, lane);
     for (int i = lane; i < ns; i += 32) c.Y[i] = c.N[i] + 2.0 * c.K1[i] + c.K3[i];
   }
   __syncthreads();
@@ -424,8 +427,7 @@ __global__ void __launch_bounds__(32 * W) debug_try_kernel(const Net net, const 
   if (warp == 0) {
     for (int i = lane; i < ns; i += 32) c.K4[i] = fma(ih, fma(-RODAS_C43, c.K3[i], c.K1[i] - c.K2[i]), c.F[i]);
     __syncwarp();
-    lu_solve<R, 1>(net, c.A, c.dinv, c.K4, nullptr, lane);
-    sherman(net, c.K4, c.U, c0, lane);
+    w_solve<R>(net, c.A, c.dinv, c.K4, c.U, c0, lane);
     try_error<R>(net, c, true, rtol, atol, lane);
   }
   __syncthreads();
@@ -444,8 +446,8 @@ __global__ void __launch_bounds__(32 * W) debug_try_kernel(const Net net, const 
 }
 
 // Cycles of each device function of a try, repeated reps times on one cell in every CTA (a tuning hook): rates,
-// F, Jacobian and w, LU, two-vector solve, one-vector solve, Sherman-Morrison, error, guard test. cycles[9] receives
-// the CTA-0 averages.
+// F, Jacobian and w, LU, solve, solve with its Sherman-Morrison correction, that correction alone, error, guard test.
+// cycles[9] receives the CTA-0 averages.
 template <int W, int R>
 __global__ void __launch_bounds__(32 * W, 16 / W) time_phases_kernel(const Net net, const double* x0, double Tc, double P,
                                                              double ha, const double* Jc, int reps,
@@ -477,10 +479,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W) time_phases_kernel(const Net n
       for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
       __syncwarp();
       u = clock64();
-      lu_solve<R, 2>(net, c.A, c.dinv, c.K1, c.U, lane);
+      lu_solve<R>(net, c.A, c.dinv, c.K1, lane);
       t = clock64();
       acc[4] += t - u;
-      lu_solve<R, 1>(net, c.A, c.dinv, c.K2, nullptr, lane);
+      w_solve<R>(net, c.A, c.dinv, c.K2, c.U, 0.5, lane);
       u = clock64();
       acc[5] += u - t;
       sherman(net, c.K2, c.U, 0.5, lane);

@@ -72,6 +72,188 @@ __device__ __forceinline__ void directional_rates(const Net& net, const Cell& c,
   if (gtid == 0) c.v[net.nr] = 0.0;
 }
 
+constexpr int PANEL = 8;  // pivots per block of the LU
+
+// ---- the FP32 LU without exchanges, blocked (PANEL pivots at a time), with a lookahead of one panel ----
+// Every entry receives its updates in ascending pivot order, as the plain path's. Per block: the block's pivot rows beyond the panel (one
+// thread per column); then warp 0 applies the block to the next panel's columns and factors that panel (one lane per
+// row, warp syncs only) while warps 1-3 apply it to the columns past the next panel, as a rank-PANEL update in 4 x 4
+// register tiles (rows and columns cyclic, so a warp's loads are broadcast or consecutive).
+
+// the trailing update of rows ke.. and columns cs.. (cs >= ke) by NT threads
+template <int NT>
+__device__ __forceinline__ void trailing_update_from(float* A, int ld, int kb, int nb, int ke, int cs, int ns, int tid) {
+  constexpr int CG = 16, RG = NT / CG;
+  const int cg = tid % CG, rg = tid / CG, m = ns - ke, mc = ns - cs;
+  for (int rb = rg; rb < m; rb += 4 * RG) {
+    for (int cb = cg; cb < mc; cb += 4 * CG) {
+      int row[4], col[4];
+      bool rok[4], cok[4];
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        rok[a] = rb + RG * a < m;
+        row[a] = ke + (rok[a] ? rb + RG * a : 0);
+        cok[a] = cb + CG * a < mc;
+        col[a] = cs + (cok[a] ? cb + CG * a : 0);
+      }
+      float acc[4][4];
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) acc[a][b] = A[row[a] * ld + col[b]];
+#pragma unroll 2
+      for (int t = 0; t < PANEL; t++) {
+        if (t < nb) {
+          float l[4], u[4];
+#pragma unroll
+          for (int a = 0; a < 4; a++) {
+            l[a] = A[row[a] * ld + kb + t];
+            u[a] = A[(kb + t) * ld + col[a]];
+          }
+#pragma unroll
+          for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int b = 0; b < 4; b++) acc[a][b] = fma(-l[a], u[b], acc[a][b]);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+          if (rok[a] && cok[b]) A[row[a] * ld + col[b]] = acc[a][b];
+    }
+  }
+}
+
+// the panel kb .. kb + nb - 1 on one warp (lane), warp-level syncs only
+__device__ __forceinline__ void panel_warp(float* A, int ld, float* dinv, int kb, int nb, int ns, int lane) {
+  const int ke = kb + nb;
+  if (lane == 0) dinv[kb] = __frcp_rn(A[kb * ld + kb]);
+  __syncwarp();
+  for (int k = kb; k < ke; k++) {
+    const float d = dinv[k];
+    float piv[PANEL];
+#pragma unroll
+    for (int jj = 1; jj < PANEL; jj++) piv[jj] = k + jj < ke ? A[k * ld + k + jj] : 0.0f;
+#pragma unroll 1
+    for (int i = k + 1 + lane; i < ns; i += 32) {
+      float* ai = A + i * ld;
+      const float l = ai[k] * d;
+      ai[k] = l;
+#pragma unroll
+      for (int jj = 1; jj < PANEL; jj++)
+        if (k + jj < ke) ai[k + jj] = fma(-l, piv[jj], ai[k + jj]);
+    }
+    // the next pivot is final now and its row is lane 0's (its first row), so lane 0 takes the reciprocal of its own
+    // write, after the row loop
+    if (lane == 0 && k + 1 < ke) dinv[k + 1] = __frcp_rn(A[(k + 1) * ld + k + 1]);
+    __syncwarp();
+  }
+}
+
+// the blocked LU with a lookahead of one panel: while warps 1-3 apply panel p to the columns past panel p + 1, warp 0
+// applies it to panel p + 1's columns and factors panel p + 1. Each entry takes its updates in ascending pivot order.
+template <int NT>
+__device__ __forceinline__ void lu_factor(const Net& net, float* A, float* dinv, int tid) {
+  const int ns = net.ns, ld = net.ld, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) panel_warp(A, ld, dinv, 0, min(PANEL, ns), ns, lane);
+  __syncthreads();
+  for (int kb = 0; kb < ns; kb += PANEL) {
+    const int ke = min(kb + PANEL, ns), nb = ke - kb;
+    if (ke == ns) break;
+    for (int j = ke + tid; j < ns; j += NT) {  // the block's pivot rows beyond the panel
+      float row[PANEL];
+#pragma unroll
+      for (int s = 0; s < PANEL; s++) row[s] = s < nb ? A[(kb + s) * ld + j] : 0.0f;
+#pragma unroll
+      for (int s = 1; s < PANEL; s++) {
+        if (s < nb) {
+          float a = row[s];
+#pragma unroll
+          for (int t = 0; t < PANEL; t++)
+            if (t < s) a = fma(-A[(kb + s) * ld + kb + t], row[t], a);
+          row[s] = a;
+          A[(kb + s) * ld + j] = a;
+        }
+      }
+    }
+    __syncthreads();
+    const int ken = min(ke + PANEL, ns);
+    if (warp == 0) {
+#pragma unroll 1
+      for (int i = ke + lane; i < ns; i += 32) {  // panel p + 1's columns, rows ke..
+        float* ai = A + i * ld;
+        float l[PANEL];
+#pragma unroll
+        for (int t = 0; t < PANEL; t++) l[t] = t < nb ? ai[kb + t] : 0.0f;
+        for (int j = ke; j < ken; j++) {
+          float acc = ai[j];
+#pragma unroll
+          for (int t = 0; t < PANEL; t++)
+            if (t < nb) acc = fma(-l[t], A[(kb + t) * ld + j], acc);
+          ai[j] = acc;
+        }
+      }
+      __syncwarp();
+      panel_warp(A, ld, dinv, ke, ken - ke, ns, lane);
+    } else {
+      trailing_update_from<NT - 32>(A, ld, kb, nb, ke, ken, ns, tid - 32);
+    }
+    __syncthreads();
+  }
+}
+
+// The forward and backward sweeps of M0^-1 on a vector in registers (a: lane l holds rows l + 32 p;
+// d: 1 / U_kk). On return a[p] * d[p] is the solution.
+template <int R>
+__device__ __forceinline__ void lu_sweep(const Net& net, const float* A, float (&a)[R], const float (&d)[R], int lane) {
+  const int ns = net.ns, ld = net.ld, last = ns - 1;
+#pragma unroll
+  for (int c = 0; c < R; c++) {  // forward: pivots 32c .. 32c + 31
+    const int k0 = 32 * c, k1 = min(k0 + 32, last);
+    if (k0 >= k1) break;
+    float m[R];
+#pragma unroll
+    for (int p = c; p < R; p++) m[p] = A[min(lane + 32 * p, last) * ld + k0];
+#pragma unroll 2
+    for (int k = k0; k < k1; k++) {
+      const float yk = __shfl_sync(FULL, a[c], k & 31);
+      float mn[R];
+#pragma unroll
+      for (int p = c; p < R; p++) mn[p] = A[min(lane + 32 * p, last) * ld + min(k + 1, last)];
+#pragma unroll
+      for (int p = c; p < R; p++) {
+        const bool act = (p > c ? true : lane > k - k0) && lane + 32 * p < ns;
+        const float mm = act ? m[p] : 0.0f;
+        a[p] = fma(-mm, yk, a[p]);
+        m[p] = mn[p];
+      }
+    }
+  }
+#pragma unroll
+  for (int c = R - 1; c >= 0; c--) {  // backward: pivots 32c + 31 .. 32c (down to 1)
+    const int k0 = 32 * c, khi = min(k0 + 31, last), klo = max(k0, 1);
+    if (khi < klo) continue;
+    float m[R];
+#pragma unroll
+    for (int p = 0; p <= c; p++) m[p] = A[min(lane + 32 * p, last) * ld + khi];
+#pragma unroll 2
+    for (int k = khi; k >= klo; k--) {
+      const float z = __shfl_sync(FULL, a[c] * d[c], k & 31);
+      float mn[R];
+#pragma unroll
+      for (int p = 0; p <= c; p++) mn[p] = A[min(lane + 32 * p, last) * ld + max(k - 1, 0)];
+#pragma unroll
+      for (int p = 0; p <= c; p++) {
+        const bool act = p < c ? true : lane < k - k0;
+        const float mm = act ? m[p] : 0.0f;
+        a[p] = fma(-mm, z, a[p]);
+        m[p] = mn[p];
+      }
+    }
+  }
+}
+
 // A (FP32, row stride ld) = -Jn off the diagonal, Dg = -Jn's diagonal (FP64), from the plain path's entry streams.
 // Two barriers.
 __device__ __forceinline__ void jacobian_mixed(const Net& net, const Cell& c, const Extra& e, int tid, int nt) {
@@ -151,19 +333,19 @@ __device__ __noinline__ void solve32(const Net& net, const Extra& e, double* y, 
   if (m > 0.0 && isfinite(m)) frexp(m, &ex);
   ex = min(max(ex, -1000), 1000);
   const double g = ldexp(1.0, -ex), ig = ldexp(1.0, ex);
-  float a[1][R], d[R];
+  float a[R], d[R];
 #pragma unroll
   for (int p = 0; p < R; p++) {
     const int i = lane + 32 * p;
-    a[0][p] = (float)(b[p] * g);
+    a[p] = (float)(b[p] * g);
     d[p] = i < ns ? e.dinv[i] : 0.0f;
   }
-  lu_sweep<R, 1, float>(net, e.A, a, d, lane);
+  lu_sweep<R>(net, e.A, a, d, lane);
   __syncwarp();
 #pragma unroll
   for (int p = 0; p < R; p++) {
     const int i = lane + 32 * p;
-    if (i < ns) y[i] = (double)(a[0][p] * d[p]) * ig;
+    if (i < ns) y[i] = (double)(a[p] * d[p]) * ig;
   }
   __syncwarp();
 }
@@ -309,7 +491,7 @@ __global__ void __launch_bounds__(32 * W, 20 / W)
       }
       scale_rows(net, e, igh, tid, nt);  // ends with a barrier
       mark(PH_RHS_JAC);
-      lu_factor<32 * W, float>(net, e.A, e.dinv, tid);
+      lu_factor<32 * W>(net, e.A, e.dinv, tid);
       mark(PH_LU);
       double worst = 0.0;
       if (warp == 0) {  // stage 1: K1 on warp 0, M0^-1 w on warp 1, then Sherman-Morrison
@@ -497,7 +679,7 @@ __global__ void __launch_bounds__(32 * W) mixed_debug_kernel(const Net net, cons
     c.U[i] = wi;
   }
   scale_rows(net, e, igh, tid, nt);
-  lu_factor<32 * W, float>(net, e.A, e.dinv, tid);
+  lu_factor<32 * W>(net, e.A, e.dinv, tid);
   if (warp == 0) {
     for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
     __syncwarp();

@@ -184,9 +184,9 @@ __device__ __noinline__ void primal_try(const Net& net, const Cell& c, const Ste
   if (warp == 0) {
     for (int i = lane; i < ns; i += 32) c.K1[i] = c.F[i];
     __syncwarp();
-    lu_solve<R, 1>(net, c.A, c.dinv, c.K1, nullptr, lane);
+    lu_solve<R>(net, c.A, c.dinv, c.K1, lane);
   } else if (warp == 1) {
-    lu_solve<R, 1>(net, c.A, c.dinv, c.U, nullptr, lane);
+    lu_solve<R>(net, c.A, c.dinv, c.U, lane);
   }
   __syncthreads();
   if (warp == 0) {
@@ -200,7 +200,7 @@ __device__ __noinline__ void primal_try(const Net& net, const Cell& c, const Ste
   }
   __syncthreads();
   if (warp == 0) {
-    lu_solve<R, 1>(net, c.A, c.dinv, c.K2, nullptr, lane);
+    lu_solve<R>(net, c.A, c.dinv, c.K2, lane);
     sherman(net, c.K2, c.U, c0, lane);
   } else {
     rhs(net, c, c.Y, false, nd, tid - 32, nt - 32, 1);
@@ -209,7 +209,7 @@ __device__ __noinline__ void primal_try(const Net& net, const Cell& c, const Ste
   if (warp == 0) {
     for (int i = lane; i < ns; i += 32) c.K3[i] = fma(ih, c.K1[i] - c.K2[i], c.F[i]);
     __syncwarp();
-    lu_solve<R, 1>(net, c.A, c.dinv, c.K3, nullptr, lane);
+    lu_solve<R>(net, c.A, c.dinv, c.K3, lane);
     sherman(net, c.K3, c.U, c0, lane);
     for (int i = lane; i < ns; i += 32) c.Y[i] = c.N[i] + 2.0 * c.K1[i] + c.K3[i];
   }
@@ -218,7 +218,7 @@ __device__ __noinline__ void primal_try(const Net& net, const Cell& c, const Ste
   if (warp == 0) {
     for (int i = lane; i < ns; i += 32) c.K4[i] = fma(ih, fma(-RODAS_C43, c.K3[i], c.K1[i] - c.K2[i]), c.F[i]);
     __syncwarp();
-    lu_solve<R, 1>(net, c.A, c.dinv, c.K4, nullptr, lane);
+    lu_solve<R>(net, c.A, c.dinv, c.K4, lane);
     sherman(net, c.K4, c.U, c0, lane);
     try_error<R>(net, c, s.t == 0.0, rtol, atol, lane);
   }
@@ -248,7 +248,7 @@ __device__ __forceinline__ void primal_update(const Net& net, const Cell& c, Ste
 // y <- M0^-T y with the factors of the LU (unit L below the diagonal, U on and above it), on one warp: U^T z = y in
 // ascending pivots (z_k = a_k / U_kk, then a_i -= U_ki z_k for i > k), then L^T x = z in descending pivots
 // (a_i -= L_ki x_k for i < k). Lane l holds rows l + 32 p; row k of the factors is read across the lanes
-// (consecutive addresses). As lu_sweep: pivots 32 at a time, the pivot's value from a register chosen at compile
+// (consecutive addresses). Pivots 32 at a time, the pivot's value from a register chosen at compile
 // time and one shuffle, and the next row loaded while the current pivot is applied; a lane whose row takes no update
 // from pivot k uses the multiplier 0 (fma(-0, z, a) = a for finite z). Each entry takes the one-pivot sweep's fma's in
 // its order.
