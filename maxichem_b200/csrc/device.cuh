@@ -376,7 +376,7 @@ __device__ __forceinline__ void jacobian_w(const Net& net, const Cell& c, double
 
 // c (8 x 8: lane 4 g + t holds row g, columns 2 t and 2 t + 1) += a (8 x 4: row g, column t) b (4 x 8: row t, column g)
 __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c0), "+d"(c1) : "d"(a), "d"(b));
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c0), "+d"(c1) : "d"(a), "d"(b));
 }
 
 __device__ __forceinline__ void pair_from(const double* p, double& a, double& b) {
