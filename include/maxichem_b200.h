@@ -267,6 +267,13 @@ int mx_set_grid(mx_solver* s, int32_t ctas_per_sm);
 int mx_debug_try(mx_solver* s, const double* x, double T, double P, double h, const double* J, double rtol,
                  double atol, double* out, void* stream);
 
+/* The call's linear algebra on a given matrix a [ns][ns] and vectors y, u [ns] (device arrays): pivoted 0 the LU without
+ * exchanges, the solve of y, and that with its Sherman-Morrison correction by u and c0; pivoted 1 the recovery's LU and
+ * solve of y. Writes to the device array out the factors [ns][ns], 1 / pivots [ns], the row order [ns], the solution
+ * [ns] and the corrected one [ns] (pivoted: the solution). No counterpart in the reference: a test hook. */
+int mx_debug_lu(mx_solver* s, const double* a, const double* y, const double* u, double c0, int32_t pivoted,
+                double* out, void* stream);
+
 /* Register a device int64[3] that later calls of this solver add their tries to: [0] the call kernel's tries, [1] those
  * that followed a rejection, [2] the recovery's tries (NULL stops counting). No counterpart in the reference: it
  * feeds the measured roofline (algorithmic FLOPs per try are a property of the network's tables). */

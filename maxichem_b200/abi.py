@@ -141,6 +141,7 @@ SIGNATURES: dict[str, tuple[Any, list[Any]]] = {
         ctypes.c_int,
         [_P, _P, ctypes.c_double, ctypes.c_double, ctypes.c_double, _P, ctypes.c_double, ctypes.c_double, _P, _P],
     ),
+    "mx_debug_lu": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_double, ctypes.c_int32, _P, _P]),
     "mx_probe_fp64": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, ctypes.POINTER(ctypes.c_double)]),
     "mx_set_precision": (ctypes.c_int, [_P, ctypes.c_int32, ctypes.c_int32, ctypes.c_double]),
     "mx_sur_create": (

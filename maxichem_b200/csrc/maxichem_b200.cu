@@ -445,6 +445,46 @@ __global__ void __launch_bounds__(32 * W) debug_try_kernel(const Net net, const 
   }
 }
 
+// The call's LU and solves, or the recovery's, on a given matrix (a test hook): out = factors [ns][ns], dinv, row
+// order, solution of y, corrected solution [ns each].
+template <int W, int R>
+__global__ void __launch_bounds__(32 * W) debug_lu_kernel(const Net net, const double* a, const double* y,
+                                                          const double* u, double c0, int pivoted, double* out) {
+  extern __shared__ double smem[];
+  const Cell c = cell_arrays(net, smem);
+  const int tid = (int)threadIdx.x, nt = 32 * W, lane = tid & 31, warp = tid >> 5, ns = net.ns, ld = net.ld;
+  int* pr = c.ints + 4;
+  for (int e = tid; e < ns * ns; e += nt) c.A[(e / ns) * ld + e % ns] = a[e];
+  for (int i = tid; i < ns; i += nt) {
+    c.K1[i] = c.K2[i] = y[i];
+    c.U[i] = u[i];
+    pr[i] = i;
+  }
+  __syncthreads();
+  if (pivoted)
+    dense_lu<W, R>(net, c, pr, tid);
+  else
+    lu<W>(net, c.A, c.dinv, tid);
+  if (warp == 0) {
+    if (pivoted) {
+      dense_solve<R>(net, c.A, c.dinv, pr, c.K1, lane);
+      for (int i = lane; i < ns; i += 32) c.K2[i] = c.K1[i];
+    } else {
+      lu_solve<R>(net, c.A, c.dinv, c.K1, lane);
+      w_solve<R>(net, c.A, c.dinv, c.K2, c.U, c0, lane);
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < ns * ns; e += nt) out[e] = c.A[(e / ns) * ld + e % ns];
+  out += ns * ns;
+  for (int i = tid; i < ns; i += nt) {
+    out[i] = c.dinv[i];
+    out[ns + i] = pr[i];
+    out[2 * ns + i] = c.K1[i];
+    out[3 * ns + i] = c.K2[i];
+  }
+}
+
 // Cycles of each device function of a try, repeated reps times on one cell in every CTA (a tuning hook): rates,
 // F, Jacobian and w, LU, solve, solve with its Sherman-Morrison correction, that correction alone, error, guard test.
 // cycles[9] receives the CTA-0 averages.
@@ -547,6 +587,7 @@ void kernels_for(mx_solver* s) {
   s->call_list = call_kernel<W, R, false, true>;
   s->recover = recover_kernel<W, R>;
   s->debug = debug_try_kernel<W, R>;
+  s->debug_lu = debug_lu_kernel<W, R>;
   s->rows_per_lane = R;
 }
 
@@ -988,6 +1029,15 @@ extern "C" int mx_debug_try(mx_solver* s, const double* x, double T, double P, d
   if (!s || !x || !out || (s->net.nj > 0 && !J)) return MX_ERR_ARGUMENT;
   DeviceScope scope(s->device);
   s->debug<<<1, 32 * s->warps, s->smem, (cudaStream_t)stream>>>(s->net, x, T, P, h, J, rtol, atol, out);
+  return cudaGetLastError() == cudaSuccess ? MX_OK : MX_ERR_CUDA;
+}
+
+extern "C" int mx_debug_lu(mx_solver* s, const double* a, const double* y, const double* u, double c0, int32_t pivoted,
+                           double* out, void* stream) {
+  if (!s || !a || !y || !u || !out) return MX_ERR_ARGUMENT;
+  DeviceScope scope(s->device);
+  cudaFuncSetAttribute((const void*)s->debug_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem);
+  s->debug_lu<<<1, 32 * s->warps, s->smem, (cudaStream_t)stream>>>(s->net, a, y, u, c0, pivoted ? 1 : 0, out);
   return cudaGetLastError() == cudaSuccess ? MX_OK : MX_ERR_CUDA;
 }
 

@@ -15,6 +15,7 @@ constexpr int WARPS = 4;  // warps per cell by default (the derivative kernels' 
 typedef void (*CallFn)(const mx::Net, const mx::CallArgs, long long*);
 typedef void (*DebugFn)(const mx::Net, const double*, double, double, double, const double*, double, double, double*);
 typedef void (*RecoverFn)(const mx::Net, const mx::CallArgs, int);
+typedef void (*DebugLuFn)(const mx::Net, const double*, const double*, const double*, double, int, double*);
 typedef void (*TimeFn)(const mx::Net, const double*, double, double, double, const double*, int, long long*);
 typedef void (*MixedFn)(const mx::Net, const mx::CallArgs, int, double, long long*);
 typedef void (*MixedDebugFn)(const mx::Net, const double*, double, double, double, const double*, double, double, int,
@@ -32,6 +33,7 @@ struct mx_solver {
   CallFn call_list = nullptr;  // the plain kernel over the cells the mixed kernel listed (a.sel)
   RecoverFn recover = nullptr;
   DebugFn debug = nullptr;
+  DebugLuFn debug_lu = nullptr;
   TimeFn timer = nullptr;
   int rows_per_lane = 0;
   size_t smem = 0;

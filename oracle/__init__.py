@@ -59,6 +59,10 @@ def library() -> ctypes.CDLL:
         lib.mxo_dense_lu.argtypes = [ctypes.c_int, P, P, P]
         lib.mxo_dense_solve.restype = None
         lib.mxo_dense_solve.argtypes = [ctypes.c_int, P, P, P, P, P]
+        lib.mxo_lu.restype = lib.mxo_lu_solve.restype = lib.mxo_sherman.restype = None
+        lib.mxo_lu.argtypes = [ctypes.c_int, P, P]
+        lib.mxo_lu_solve.argtypes = [ctypes.c_int, P, P, P]
+        lib.mxo_sherman.argtypes = [ctypes.c_int, P, P, D]
         lib.mxo_screen.restype = ctypes.c_int
         lib.mxo_screen.argtypes = [P, P, D, D, D, P, P]
         lib.mxo_threads.restype = ctypes.c_int
@@ -177,6 +181,27 @@ def dense_solve(a: np.ndarray, dinv: np.ndarray, pr: np.ndarray, y: np.ndarray) 
     work = np.empty_like(y)
     library().mxo_dense_solve(len(y), _p(_f64(a)), _p(_f64(dinv)), _p(np.ascontiguousarray(pr, np.int32)), _p(y),
                               _p(work))
+    return y
+
+
+def lu(a: np.ndarray) -> tuple[np.ndarray, np.ndarray]:
+    """The plain path's LU without exchanges: factors, 1 / pivots."""
+    a = _f64(a).copy()
+    dinv = np.empty(a.shape[0])
+    library().mxo_lu(a.shape[0], _p(a), _p(dinv))
+    return a, dinv
+
+
+def lu_solve(a: np.ndarray, dinv: np.ndarray, y: np.ndarray) -> np.ndarray:
+    y = _f64(y).copy()
+    library().mxo_lu_solve(len(y), _p(_f64(a)), _p(_f64(dinv)), _p(y))
+    return y
+
+
+def sherman(y: np.ndarray, u: np.ndarray, c0: float) -> np.ndarray:
+    """y + c0 (sum y) u."""
+    y = _f64(y).copy()
+    library().mxo_sherman(len(y), _p(y), _p(_f64(u)), c0)
     return y
 
 

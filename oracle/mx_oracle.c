@@ -242,6 +242,10 @@ static void lu_solve(int ns, const double* A, const double* dinv, double* y) {
   for (int i = 0; i < ns; i++) y[i] = y[i] * dinv[i];
 }
 
+/* The plain path's LU and solve, by themselves. */
+void mxo_lu(int ns, double* A, double* dinv) { lu_factor(ns, A, dinv); }
+void mxo_lu_solve(int ns, const double* A, const double* dinv, double* y) { lu_solve(ns, A, dinv, y); }
+
 /* ---- step control (common.cuh:90-133) ---- */
 
 typedef struct {
@@ -289,6 +293,8 @@ static void sherman(int ns, double* y, const double* u, double c0) {
   const double s = lane_sum(y, ns) * c0;
   for (int i = 0; i < ns; i++) y[i] = fma(s, u[i], y[i]);
 }
+
+void mxo_sherman(int ns, double* y, const double* u, double c0) { sherman(ns, y, u, c0); }
 
 /* ---- guard (guard.cuh:13-108) ----
  * Every sum runs over the species in network order, as the reference's one thread per cell adds them. */
