@@ -101,7 +101,8 @@ typedef struct mx_network {
   int32_t sv_piece, n_pieces;
   const int32_t* sv_row_ptr;     /* [ns + 1] */
   /* Per-thread streams of the same sums for the call kernel's thread groups (maxichem_b200/tables.py
-   * thread_streams): [0] the CTA of 128 threads, [1] its last 96 threads. Word q of thread t at q * threads + t. */
+   * thread_streams): [0] the CTA of 128 threads, [1] its last 96 threads. Word q of thread t at q * threads + t. The
+   * kernels read both S v streams and the CTA's Jacobian stream; its last threads' one is only checked. */
   int32_t stream_threads[2];
   int32_t sv_rounds[2], sv_nrows[2], jac_rounds[2], jac_nents[2];
   const uint16_t* sv_stream[2];  /* reaction | code << 11 | end << 13 (padding: nr) */

@@ -552,7 +552,8 @@ __device__ __forceinline__ double pick(const double (&a)[R], int idx) {
 // one-pivot sweep's fma's in its order, four pivots at a time: their four values are gathered from their lanes, every
 // lane solves the 4 x 4 block alike (its entries are broadcast reads) and applies the four to its rows, so four
 // pivots cost one shuffle latency instead of four; the matrix's last rows past a multiple of four go one by one. One
-// warp issues it, so its instructions and their latencies are the time: 8,500 cycles at 69 species.
+// warp issues it, so its instructions and their latencies are the time: 8,600 cycles at 69 species, one pivot at a time
+// 10,700.
 // Not inlined: the call kernel solves at four places, and one copy of the code keeps the instruction cache warm; the
 // vector and the matrix are offsets into shared memory, so that its accesses stay shared ones.
 // With oU >= 0 the Sherman-Morrison correction of W = M0 - w 1^T follows (sherman's operations).

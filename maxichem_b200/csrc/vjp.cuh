@@ -72,7 +72,7 @@ constexpr int ADJ_CHUNK = 64;  // cells per chunk of the rate table's partial su
 
 // Cells of a queue item for a batch of so many chunks on `slots` resident CTAs: a chunk where each CTA gets at least
 // four, so that the queue evens out cells of different step counts, else one cell, whose contribution waits in
-// 3 nr doubles of its own. 4,096 cells of 69 species: 64 cells an item keep 64 of the 444 CTAs busy, 239 ms; one, 48 ms.
+// 3 nr doubles of its own. 4,096 cells of 69 species: 64 cells an item keep 64 of the 444 CTAs busy, 239 ms; one, 44 ms.
 inline int adjoint_run(int64_t nchunks, int64_t slots) { return nchunks < 4 * slots ? 1 : ADJ_CHUNK; }
 
 __device__ __forceinline__ double* adj_kbar(const Net& net, double* sl) { return sl; }
