@@ -370,9 +370,9 @@ __device__ __forceinline__ void jacobian_w(const Net& net, const Cell& c, double
 // each, in registers; then warp 0 updates and factors the next diagonal block while the other warps update the rest.
 // What bounds it is the chain of the diagonal blocks (69 pivots of a reciprocal, a product, an fma and a shuffle) and
 // shared-memory bandwidth: 69 species, 26,300 cycles with one cell an SM, 39,900 with four that all factor at once (a
-// factorisation in 4 x 4 register tiles 60,000 and 76,500). The loops are kept rolled where they can be: the whole try is 60 KB of code,
-// and unrolled forms that are faster alone (the diagonal block's pivots, 8-pivot solves) made the call 13 % slower with
-// four cells an SM, by instruction fetch.
+// factorisation in 4 x 4 register tiles 60,000 and 76,500). The loops are kept rolled where they can be: the whole try
+// is 60 KB of code, and unrolled forms that are faster alone (the diagonal block's pivots, 8-pivot solves) made the
+// call 13 % slower with four cells an SM, by instruction fetch.
 
 // c (8 x 8: lane 4 g + t holds row g, columns 2 t and 2 t + 1) += a (8 x 4: row g, column t) b (4 x 8: row t, column g)
 __device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
